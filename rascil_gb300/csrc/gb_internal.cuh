@@ -27,7 +27,8 @@ namespace gb {
 constexpr double kSpeedOfLight = 299792458.0;  // rascil/phyconst.py:6
 constexpr int kThreads = 256;                   // block size of the tile kernels
 constexpr int kWarps = kThreads / 32;
-constexpr int kChunkItems = 256;                // items per work chunk
+constexpr int kChunkItems = 256;                // items per work chunk (FP32 form)
+constexpr int kChunkItems64 = 64;               // and in the FP64 form
 constexpr int kMaxSupport = 16;
 constexpr int kMaxQuad = 48;                    // Gauss-Legendre nodes (half interval)
 constexpr int kMaxSlab = 128;                   // w-planes per bucket slab
@@ -48,6 +49,7 @@ struct Geom {
   int nplanes;
   int T;             // uv tile side (cells)
   int S;             // w-planes per bucket slab
+  int chunk;         // items per work chunk (at most)
   int ntu, ntv, nslabs;
   int64_t nbuckets;
   int64_t R;         // rows
@@ -89,7 +91,7 @@ template <> struct Traits<double> {
   using Item = ItemD;
 };
 
-// A unit of work for the tile kernels: up to kChunkItems consecutive items
+// A unit of work for the tile kernels: up to Geom::chunk consecutive items
 // of one bucket.
 struct Chunk {
   uint32_t begin, end, bucket, pad;

@@ -4,7 +4,8 @@
 //                           apply flags, weights, the pol-frame matrix and the
 //                           w-centring rotation; sum the weights per pol.
 // Per batch of w-planes:
-//             k_grid        one CTA per work chunk (<= 256 items of one
+//             k_grid        (FP32 form; the FP64 form's is k_grid64, gb_fp64.cu)
+//                           one CTA per work chunk (<= 256 items of one
 //                           (slab, tile) bucket): the tile's sub-grid lives in
 //                           shared memory, each warp spreads one item at a
 //                           time over its W x W support (kernel values per
@@ -125,21 +126,11 @@ __global__ void __launch_bounds__(kThreads)
 __device__ __forceinline__ void grid_add(float2 *dst, float re, float im) {
   atomicAdd(dst, make_float2(re, im));
 }
-__device__ __forceinline__ void grid_add(double2 *dst, double re, double im) {
-  atomicAdd(&dst->x, re);
-  atomicAdd(&dst->y, im);
-}
 // Two adjacent cells (dst 16-byte aligned): one vector atomic in FP32.
 __device__ __forceinline__ void grid_add2(float2 *dst, float re0, float im0, float re1,
                                           float im1) {
   atomicAdd(reinterpret_cast<float4 *>(dst), make_float4(re0, im0, re1, im1));
 }
-__device__ __forceinline__ void grid_add2(double2 *dst, double re0, double im0, double re1,
-                                          double im1) {
-  grid_add(dst, re0, im0);
-  grid_add(dst + 1, re1, im1);
-}
-
 // Slab range [s_lo, s_hi] whose items reach planes [b0, b0 + nb).
 __device__ __forceinline__ void batch_slabs(const Geom &g, int b0, int nb, int &s_lo,
                                             int &s_hi) {
@@ -150,36 +141,9 @@ __device__ __forceinline__ void batch_slabs(const Geom &g, int b0, int nb, int &
 
 // Fixed-point accumulation for the shared-memory sub-grid: integer shared
 // atomics are native, floating-point ones are not.  Each chunk gets its own
-// scale (2^30 or 2^61 over the chunk's sum of |value|), so the integer sums
-// can neither overflow nor lose more than one part in 2^30 of that bound.
-template <typename R> struct FixedAcc;
-template <> struct FixedAcc<float> {
-  using T = int;
-  using T2 = int2;
-  static constexpr double kOne = 1073741824.0;  // 2^30
-};
-template <> struct FixedAcc<double> {
-  using T = long long;
-  using T2 = longlong2;
-  static constexpr double kOne = 2305843009213693952.0;  // 2^61
-};
-__device__ __forceinline__ int to_fixed(float v) { return __float2int_rn(v); }
-__device__ __forceinline__ long long to_fixed(double v) { return __double2ll_rn(v); }
-__device__ __forceinline__ void fixed_add(int *p, int v) { atomicAdd(p, v); }
-__device__ __forceinline__ void fixed_add(long long *p, long long v) {
-  atomicAdd(reinterpret_cast<unsigned long long *>(p), static_cast<unsigned long long>(v));
-}
-
-// Shared memory of the tile gridder: the fixed-point sub-grid (2 NP planes
-// of the plan's tile layout), then, in the FP32 form, the per-chunk cache of
-// every item's kernel values {loc, ku[W], kv[W], kw[W]} and scaled values.
-template <typename R> struct GridSmem;
-template <> struct GridSmem<float> {
-  static constexpr bool kCache = true;
-};
-template <> struct GridSmem<double> {
-  static constexpr bool kCache = false;
-};
+// scale (2^30 over the chunk's sum of |value|), so the integer sums can
+// neither overflow nor lose more than one part in 2^30 of that bound.
+constexpr float kFixedOne = 1073741824.0f;  // 2^30
 
 // The FP32 gridder's spread in integer arithmetic.  For sub-grid chunks
 // the item cache holds every item's v kernel values in Q31 (round(kv 2^31),
@@ -314,30 +278,28 @@ __device__ __forceinline__ void spread_fixed(const LaneMap<NP, AW> &lm, int warp
 }
 
 // Grid one work chunk (up to kChunkItems items of one (w-slab, uv tile)
-// bucket) into the planes [b0, b0 + nb) of `grid`: spread every item over
-// its W x W support in the shared sub-grid, plane by plane, then flush the
-// sub-grid to HBM with float2 atomics and leave it zeroed.  `acc` must be all
-// zero on entry (it is on exit); kc / cc are the FP32 item cache; s_red,
-// s_scale and s_first (kMaxSlab + 1 entries) are block-shared scratch.
-// Every thread of the block calls it.
-template <typename R, int NP, int AW>
+// bucket) into the planes [b0, b0 + nb) of `grid` (FP32 form; k_grid64 is the
+// FP64 form's): spread every item over its W x W support in the shared
+// sub-grid (2 NP planes of the plan's tile layout), plane by plane, then
+// flush the sub-grid to HBM with vector atomics and leave it zeroed.  `acc`
+// must be all zero on entry (it is on exit); kc / cc are the item cache
+// ({loc, ku[W], kv[W], kw[W]} and scaled values per item); s_red, s_scale and
+// s_first (kMaxSlab + 1 entries) are block-shared scratch.  Every thread of
+// the block calls it.
+template <int NP, int AW>
 __device__ __forceinline__ void grid_chunk(
-    const Geom &g, const typename Traits<R>::Item *__restrict__ items,
-    const typename Traits<R>::C *__restrict__ cvis, const Chunk ch, int b0, int nb,
-    typename Traits<R>::C *__restrict__ grid, typename FixedAcc<R>::T *acc, R *kc,
-    typename Traits<R>::C *cc, R *s_red, R *s_scale, int *s_first) {
-  using C = typename Traits<R>::C;
-  using A = typename FixedAcc<R>::T;
+    const Geom &g, const ItemF *__restrict__ items, const float2 *__restrict__ cvis,
+    const Chunk ch, int b0, int nb, float2 *__restrict__ grid, int *acc, float *kc, float2 *cc,
+    float *s_red, float *s_scale, int *s_first) {
   using LM = LaneMap<NP, AW>;
-  constexpr bool kCache = GridSmem<R>::kCache;
   const int W = g.W, T = g.T;
   const TileLayout L = tile_layout(T, W, NP);
   constexpr int KS = kcache_stride(AW);  // item cache: loc | ku[AW] | kv[AW] | kw[AW]
   const int SW = L.SW, SW2 = SW * SW;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const LM lm(lane);
-  const R scale_u = (R)2 / (R)W;
-  const R beta = (R)g.beta;
+  const float scale_u = 2.f / (float)W;
+  const float beta = (float)g.beta;
   const int ntiles = g.ntu * g.ntv;
   const size_t plane = (size_t)g.ngx * g.ngy;
   {
@@ -354,19 +316,19 @@ __device__ __forceinline__ void grid_chunk(
     if (k_lo >= k_hi) return;  // (block-uniform) no item reaches this batch's planes
     const int n = (int)(ch.end - ch.begin);
     const bool direct = n * W * W < SW2;
-    // chunk scale for the fixed-point sub-grid: 2^k / sum_j max |component|,
-    // summed in the form's precision (the FP32 form: a sum low by a few
-    // parts in 10^7 at most, against the factor-2 headroom of the 2^30
-    // bound in int32, so no cell sum can overflow)
-    R scale = (R)0, inv = (R)0;
+    // chunk scale for the fixed-point sub-grid: 2^30 / sum_j max |component|,
+    // summed in FP32 (a sum low by a few parts in 10^7 at most, against the
+    // factor-2 headroom of the 2^30 bound in int32, so no cell sum can
+    // overflow)
+    float scale = 0.f, inv = 0.f;
     if (!direct) {
-      R m = (R)0;
+      float m = 0.f;
       for (uint32_t j = ch.begin + threadIdx.x; j < ch.end; j += kThreads) {
-        R mj = (R)0;
+        float mj = 0.f;
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
-          const C v = cvis[(size_t)j * NP + p];
-          mj = fmax(mj, fmax(fabs(v.x), fabs(v.y)));
+          const float2 v = cvis[(size_t)j * NP + p];
+          mj = fmaxf(mj, fmaxf(fabsf(v.x), fabsf(v.y)));
         }
         m += mj;
       }
@@ -375,11 +337,10 @@ __device__ __forceinline__ void grid_chunk(
       __syncthreads();
       // one thread forms the scale and its inverse
       if (threadIdx.x == 0) {
-        R S = (R)0;
+        float S = 0.f;
         for (int w = 0; w < kWarps; ++w) S += s_red[w];
-        constexpr R kOne = (R)FixedAcc<R>::kOne, kInvOne = (R)(1.0 / FixedAcc<R>::kOne);
-        s_scale[0] = S > (R)0 ? kOne / S : (R)0;
-        s_scale[1] = S > (R)0 ? S * kInvOne : (R)0;
+        s_scale[0] = S > 0.f ? kFixedOne / S : 0.f;
+        s_scale[1] = S > 0.f ? S * (1.f / kFixedOne) : 0.f;
       }
       __syncthreads();
       scale = s_scale[0];
@@ -396,117 +357,69 @@ __device__ __forceinline__ void grid_chunk(
       if (jj == n - 1)
         for (int q = lk + 1; q <= g.S; ++q) s_first[q] = n;
     }
-    if constexpr (!kCache) __syncthreads();
-    if constexpr (kCache) {
-      const R f = direct ? (R)1 : scale;
-      for (int jj = threadIdx.x; jj < n; jj += kThreads) {
-        const auto it = items[ch.begin + jj];
-        R *c = kc + jj * KS;
-        c[0] = __uint_as_float(it.loc);
+    const float f = direct ? 1.f : scale;
+    for (int jj = threadIdx.x; jj < n; jj += kThreads) {
+      const ItemF it = items[ch.begin + jj];
+      float *c = kc + jj * KS;
+      c[0] = __uint_as_float(it.loc);
 #pragma unroll
-        for (int a = 0; a < AW; ++a) {
-          const bool in = a < W;
-          c[4 + a] = in ? es_kernel(((R)a - it.du) * scale_u, beta) : (R)0;
-          // v values: float for direct chunks, Q31 for the sub-grid spread
-          const R kv = in ? es_kernel(((R)a - it.dv) * scale_u, beta) : (R)0;
-          c[4 + AW + a] = direct ? kv : __int_as_float(kernel_q31(kv));
-          c[4 + 2 * AW + a] = in ? (g.do_w ? es_kernel(((R)a - it.dwf) * scale_u, beta) : (R)1)
-                                 : (R)0;
-        }
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          C v = cvis[(size_t)(ch.begin + jj) * NP + p];
-          v.x *= f;
-          v.y *= f;
-          cc[jj * NP + p] = v;
-        }
+      for (int a = 0; a < AW; ++a) {
+        const bool in = a < W;
+        c[4 + a] = in ? es_kernel(((float)a - it.du) * scale_u, beta) : 0.f;
+        // v values: float for direct chunks, Q31 for the sub-grid spread
+        const float kv = in ? es_kernel(((float)a - it.dv) * scale_u, beta) : 0.f;
+        c[4 + AW + a] = direct ? kv : __int_as_float(kernel_q31(kv));
+        c[4 + 2 * AW + a] = in ? (g.do_w ? es_kernel(((float)a - it.dwf) * scale_u, beta) : 1.f)
+                               : 0.f;
       }
-      __syncthreads();
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        float2 v = cvis[(size_t)(ch.begin + jj) * NP + p];
+        v.x *= f;
+        v.y *= f;
+        cc[jj * NP + p] = v;
+      }
     }
+    __syncthreads();
     for (int k = k_lo; k < k_hi; ++k) {
-      C *gplane = grid + (size_t)(k - b0) * NP * plane;
+      float2 *gplane = grid + (size_t)(k - b0) * NP * plane;
       const int lk_lo = max(0, k - kbase - W + 1), lk_hi = min(g.S - 1, k - kbase);
-      const uint32_t j_lo = ch.begin + (uint32_t)s_first[lk_lo];
-      const uint32_t j_hi = lk_lo <= lk_hi ? ch.begin + (uint32_t)s_first[lk_hi + 1] : j_lo;
-      if constexpr (kCache) {
-        if (!direct)
-          spread_fixed<NP, AW>(lm, warp, W, T, k, kbase, (int)(j_lo - ch.begin),
-                               (int)(j_hi - ch.begin), kc, cc, acc, L);
-      }
-      for (uint32_t j = j_lo + warp; j < j_hi && (!kCache || direct); j += kWarps) {
-        const int jj = (int)(j - ch.begin);
-        R fw, ku, kv_lane = (R)0;
-        uint32_t loc;
-        C c[LM::NPL];
-        if constexpr (kCache) {
-          const R *kj = kc + jj * KS;
-          loc = __float_as_uint(kj[0]);
-          const int aw = k - (kbase + (int)((loc >> 16) & 0xffu));
-          if (aw < 0 || aw >= W) continue;
-          fw = kj[4 + 2 * AW + aw];
-          ku = kj[4 + lm.a];  // zero for a >= W
-          if (lane >= 16 && lane - 16 < W) kv_lane = kj[4 + AW + lane - 16];
-#pragma unroll
-          for (int i = 0; i < LM::NPL; ++i) {
-            c[i] = cc[jj * NP + lm.pol(i)];
-            c[i].x *= fw;
-            c[i].y *= fw;
-          }
-        } else {
-          const auto it = items[j];
-          loc = it.loc;
-          const int aw = k - (kbase + (int)((it.loc >> 16) & 0xffu));
-          if (aw < 0 || aw >= W) continue;
-          fw = g.do_w ? es_kernel(((R)aw - it.dwf) * scale_u, beta) : (R)1;
-          // lanes 0..15 hold the u kernel values, 16..31 the v values
-          if (lane < 16) {
-            if (lane < W) kv_lane = es_kernel(((R)lane - it.du) * scale_u, beta);
-          } else if (lane - 16 < W) {
-            kv_lane = es_kernel(((R)(lane - 16) - it.dv) * scale_u, beta);
-          }
-          ku = __shfl_sync(0xffffffffu, kv_lane, lm.a);
-#pragma unroll
-          for (int i = 0; i < LM::NPL; ++i) {
-            c[i] = cvis[(size_t)j * NP + lm.pol(i)];
-            const R f = fw * (direct ? (R)1 : scale);
-            c[i].x *= f;
-            c[i].y *= f;
-          }
-        }
-        const int lu = (int)(loc & 0xffu), lv = (int)((loc >> 8) & 0xffu);
+      const int j_lo = s_first[lk_lo];
+      const int j_hi = lk_lo <= lk_hi ? s_first[lk_hi + 1] : j_lo;
+      if (!direct) spread_fixed<NP, AW>(lm, warp, W, T, k, kbase, j_lo, j_hi, kc, cc, acc, L);
+      for (int jj = j_lo + warp; jj < j_hi && direct; jj += kWarps) {
+        const float *kj = kc + jj * KS;
+        const uint32_t loc = __float_as_uint(kj[0]);
+        const int aw = k - (kbase + (int)((loc >> 16) & 0xffu));
+        if (aw < 0 || aw >= W) continue;
         // the lane's column kernel value folded into its values once per
         // item and plane: a support row then costs one multiply per part
+        const float fw = kj[4 + 2 * AW + aw], ku = kj[4 + lm.a];  // zero for a >= W
+        float kv_lane = 0.f;
+        if (lane >= 16 && lane - 16 < W) kv_lane = kj[4 + AW + lane - 16];
+        float2 c[LM::NPL];
 #pragma unroll
         for (int i = 0; i < LM::NPL; ++i) {
-          c[i].x *= ku;
-          c[i].y *= ku;
+          c[i] = cc[jj * NP + lm.pol(i)];
+          c[i].x = c[i].x * fw * ku;
+          c[i].y = c[i].y * fw * ku;
         }
+        const int lu = (int)(loc & 0xffu), lv = (int)((loc >> 8) & 0xffu);
         constexpr int kMaxRows = (AW + LM::RS - 1) / LM::RS;  // W <= AW: unrolled, predicated
-        const int cell0 = (lv + lm.r0) * L.pitch + lu + lm.a;
 #pragma unroll
         for (int r = 0; r < kMaxRows; ++r) {
           const int b = lm.r0 + r * LM::RS;
-          const R kv = __shfl_sync(0xffffffffu, kv_lane, 16 + min(b, W - 1));
+          const float kv = __shfl_sync(0xffffffffu, kv_lane, 16 + min(b, W - 1));
           if (b < W && lm.a < W) {
-            if (direct) {
-              int p = tu * T + lu + lm.a;
-              if (p >= g.ngx) p -= g.ngx;
-              int q = tv * T + lv + b;
-              if (q >= g.ngy) q -= g.ngy;
-              const R f = ((p + q) & 1) ? -kv : kv;
+            int p = tu * T + lu + lm.a;
+            if (p >= g.ngx) p -= g.ngx;
+            int q = tv * T + lv + b;
+            if (q >= g.ngy) q -= g.ngy;
+            const float f = ((p + q) & 1) ? -kv : kv;
 #pragma unroll
-              for (int i = 0; i < LM::NPL; ++i)
-                grid_add(&gplane[lm.pol(i) * plane + (size_t)q * g.ngx + p], f * c[i].x,
-                         f * c[i].y);
-            } else {
-              const int cell = cell0 + r * LM::RS * L.pitch;
-#pragma unroll
-              for (int i = 0; i < LM::NPL; ++i) {
-                const int pl = lm.pol(i);
-                fixed_add(&acc[pl * L.plane + cell], to_fixed(kv * c[i].x));
-                fixed_add(&acc[(NP + pl) * L.plane + cell], to_fixed(kv * c[i].y));
-              }
-            }
+            for (int i = 0; i < LM::NPL; ++i)
+              grid_add(&gplane[lm.pol(i) * plane + (size_t)q * g.ngx + p], f * c[i].x,
+                       f * c[i].y);
           }
         }
       }
@@ -526,21 +439,19 @@ __device__ __forceinline__ void grid_chunk(
           while (p >= g.ngx) p -= g.ngx;
           int q = tv * T + y;
           while (q >= g.ngy) q -= g.ngy;
-          const R sgn = ((p + q) & 1) ? -inv : inv;  // the pair's second cell: -sgn
+          const float sgn = ((p + q) & 1) ? -inv : inv;  // the pair's second cell: -sgn
 #pragma unroll
           for (int pol = 0; pol < NP; ++pol) {
-            // the pair as one 8-byte (FP32 form) or 16-byte (FP64 form)
-            // shared access: cell is even, and so are the pitch and the
-            // plane stride
-            using A2 = typename FixedAcc<R>::T2;
-            A2 *are = reinterpret_cast<A2 *>(acc + pol * L.plane + cell);
-            A2 *aim = reinterpret_cast<A2 *>(acc + (NP + pol) * L.plane + cell);
-            const A2 re = *are, im = *aim;
+            // the pair as one 8-byte shared access: cell is even, and so are
+            // the pitch and the plane stride
+            int2 *are = reinterpret_cast<int2 *>(acc + pol * L.plane + cell);
+            int2 *aim = reinterpret_cast<int2 *>(acc + (NP + pol) * L.plane + cell);
+            const int2 re = *are, im = *aim;
             if ((re.x | re.y | im.x | im.y) != 0) {
-              *are = A2{0, 0};
-              *aim = A2{0, 0};
-              grid_add2(&gplane[pol * plane + (size_t)q * g.ngx + p], sgn * (R)re.x,
-                        sgn * (R)im.x, -sgn * (R)re.y, -sgn * (R)im.y);
+              *are = make_int2(0, 0);
+              *aim = make_int2(0, 0);
+              grid_add2(&gplane[pol * plane + (size_t)q * g.ngx + p], sgn * (float)re.x,
+                        sgn * (float)im.x, -sgn * (float)re.y, -sgn * (float)im.y);
             }
           }
         }
@@ -550,19 +461,16 @@ __device__ __forceinline__ void grid_chunk(
   }
 }
 
-template <typename R, int NP, int AW>
+template <int NP, int AW>
 __global__ void __launch_bounds__(kThreads)
-    k_grid(const Geom g, const typename Traits<R>::Item *__restrict__ items,
-           const typename Traits<R>::C *__restrict__ cvis, const Chunk *__restrict__ chunks,
-           const uint32_t *__restrict__ chunk_off, int b0, int nb,
-           typename Traits<R>::C *__restrict__ grid, uint32_t *__restrict__ counter) {
-  using C = typename Traits<R>::C;
-  using A = typename FixedAcc<R>::T;
+    k_grid(const Geom g, const ItemF *__restrict__ items, const float2 *__restrict__ cvis,
+           const Chunk *__restrict__ chunks, const uint32_t *__restrict__ chunk_off, int b0, int nb,
+           float2 *__restrict__ grid, uint32_t *__restrict__ counter) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  A *acc = reinterpret_cast<A *>(smem_raw);  // [re pols | im pols][SW][pitch]
+  int *acc = reinterpret_cast<int *>(smem_raw);  // [re pols | im pols][SW][pitch]
   const TileLayout L = tile_layout(g.T, g.W, NP);
-  R *kc = reinterpret_cast<R *>(acc + 2 * NP * L.plane);  // [kChunkItems][kcache_stride]
-  C *cc = reinterpret_cast<C *>(kc + kChunkItems * kcache_stride(AW));  // [kChunkItems][NP]
+  float *kc = reinterpret_cast<float *>(acc + 2 * NP * L.plane);  // [kChunkItems][kcache_stride]
+  float2 *cc = reinterpret_cast<float2 *>(kc + kChunkItems * kcache_stride(AW));  // [kChunkItems][NP]
   const int ntiles = g.ntu * g.ntv;
   int s_lo, s_hi;
   batch_slabs(g, b0, nb, s_lo, s_hi);
@@ -570,15 +478,15 @@ __global__ void __launch_bounds__(kThreads)
   const uint32_t c_end = chunk_off[(int64_t)(s_hi + 1) * ntiles];
   for (int i = threadIdx.x; i < 2 * NP * L.plane; i += kThreads) acc[i] = 0;
   __shared__ uint32_t s_ci;
-  __shared__ R s_red[kWarps];
-  __shared__ R s_scale[2];
+  __shared__ float s_red[kWarps];
+  __shared__ float s_scale[2];
   __shared__ int s_first[kMaxSlab + 1];
   for (;;) {
     if (threadIdx.x == 0) s_ci = c_begin + atomicAdd(counter, 1u);
     __syncthreads();
     const uint32_t ci = s_ci;
     if (ci >= c_end) break;
-    grid_chunk<R, NP, AW>(g, items, cvis, chunks[ci], b0, nb, grid, acc, kc, cc, s_red, s_scale,
+    grid_chunk<NP, AW>(g, items, cvis, chunks[ci], b0, nb, grid, acc, kc, cc, s_red, s_scale,
                           s_first);
   }
 }
@@ -681,19 +589,12 @@ int run_fft(gb_plan *p, int nb, void *data, int dir, cudaStream_t s) {
   return GB_OK;
 }
 
-// Shared memory of k_grid / k_degrid: 2 NP planes of 4- or 8-byte words.
-size_t tile_smem_bytes(const gb_plan *p) {
-  const TileLayout L = tile_layout(p->g.T, p->g.W, p->g.NP);
-  return (size_t)2 * p->g.NP * L.plane * real_bytes(p->precision);
-}
-
-// k_grid: the sub-grid plus, in the FP32 form, the per-chunk item cache.
+// Shared memory of k_grid: 2 NP planes of 4-byte words and the item cache.
 size_t grid_smem_bytes(const gb_plan *p) {
-  size_t b = tile_smem_bytes(p);
-  if (p->precision == GB_FP32)
-    b += (size_t)kChunkItems *
-         (kcache_stride(group_lanes(p->g.W)) * sizeof(float) + p->g.NP * sizeof(float2));
-  return b;
+  const TileLayout L = tile_layout(p->g.T, p->g.W, p->g.NP);
+  return (size_t)2 * p->g.NP * L.plane * sizeof(int) +
+         (size_t)kChunkItems *
+             (kcache_stride(group_lanes(p->g.W)) * sizeof(float) + p->g.NP * sizeof(float2));
 }
 
 // The invert driver in steps (a batch of plans interleaves them across
@@ -762,28 +663,31 @@ static void grid_counts(const gb_plan *p, int bi, double *bytes, double *updates
 template <typename R, int NP>
 static int inv_grid_impl(gb_plan *p, int bi, cudaStream_t s) {
   using C = typename Traits<R>::C;
-  using Item = typename Traits<R>::Item;
   const Geom &g = p->g;
   char *tmp = p->ws + p->off_temp;
   C *grid = reinterpret_cast<C *>(tmp + p->c_grid);
   const C *cvis = reinterpret_cast<const C *>(tmp + p->c_cvis);
   uint32_t *counters = p->at<uint32_t>(p->off_counters);
-  const Item *items = p->at<Item>(p->off_items);
-  const Chunk *chunks = p->at<Chunk>(p->off_chunks);
-  const uint32_t *chunk_off = p->at<uint32_t>(p->off_chunk_off);
   const int b0 = bi * g.B, nb = std::min(g.B, g.nplanes - b0);
-  const size_t smem = grid_smem_bytes(p);
   double bytes = 0.0, updates = 0.0;
   if (prof_on()) grid_counts<R, NP>(p, bi, &bytes, &updates);
   ProfScope ps(kProfGrid, s, bytes, updates);
-  if (group_lanes(g.W) == 8)
-    k_grid<R, NP, 8><<<p->grid_blocks, kThreads, smem, s>>>(g, items, cvis, chunks, chunk_off,
-                                                            b0, nb, grid, counters + bi);
-  else
-    k_grid<R, NP, 16><<<p->grid_blocks, kThreads, smem, s>>>(g, items, cvis, chunks, chunk_off,
-                                                             b0, nb, grid, counters + bi);
-  GB_LAUNCH_CHECK("k_grid");
-  return GB_OK;
+  if constexpr (std::is_same<R, double>::value) {
+    return launch_grid64(p, b0, nb, cvis, grid, counters + bi, s);
+  } else {
+    const ItemF *items = p->at<ItemF>(p->off_items);
+    const Chunk *chunks = p->at<Chunk>(p->off_chunks);
+    const uint32_t *chunk_off = p->at<uint32_t>(p->off_chunk_off);
+    const size_t smem = grid_smem_bytes(p);
+    if (group_lanes(g.W) == 8)
+      k_grid<NP, 8><<<p->grid_blocks, kThreads, smem, s>>>(g, items, cvis, chunks, chunk_off, b0,
+                                                           nb, grid, counters + bi);
+    else
+      k_grid<NP, 16><<<p->grid_blocks, kThreads, smem, s>>>(g, items, cvis, chunks, chunk_off, b0,
+                                                            nb, grid, counters + bi);
+    GB_LAUNCH_CHECK("k_grid");
+    return GB_OK;
+  }
 }
 
 template <typename R, int NP>
@@ -930,7 +834,7 @@ __global__ void __launch_bounds__(kThreads)
     if (w >= total) break;
     const GridJob &jb = jobs.job[s_j];
     const uint32_t ci = s_cbeg[s_j] + (w - s_wbeg[s_j]);
-    grid_chunk<float, NP, AW>(jb.g, reinterpret_cast<const ItemF *>(jb.items),
+    grid_chunk<NP, AW>(jb.g, reinterpret_cast<const ItemF *>(jb.items),
                               reinterpret_cast<const float2 *>(jb.cvis), jb.chunks[ci], jb.b0,
                               jb.nb, reinterpret_cast<float2 *>(jb.grid), acc, kc, cc, s_red,
                               s_scale, s_first);
@@ -1032,14 +936,13 @@ int run_ms2dirty(gb_plan *p, const void *vis, int npv, const void *wgt, const vo
 #undef GB_CASE
 }
 
-template <typename R, int NP, int AW>
+template <int NP, int AW>
 static int setup_grid_aw(gb_plan *p) {
   const size_t smem = grid_smem_bytes(p);
-  GB_CUDA(cudaFuncSetAttribute(k_grid<R, NP, AW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem));
+  auto k = k_grid<NP, AW>;
+  GB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
-  GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_grid<R, NP, AW>, kThreads,
-                                                        smem));
+  GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem));
   if (per_sm < 1) {
     set_error("k_grid cannot launch with %zu bytes of shared memory", smem);
     return GB_ERR_INVALID_ARG;
@@ -1048,23 +951,16 @@ static int setup_grid_aw(gb_plan *p) {
   return GB_OK;
 }
 
-template <typename R, int NP>
-static int setup_grid_impl(gb_plan *p) {
-  return group_lanes(p->g.W) == 8 ? setup_grid_aw<R, NP, 8>(p) : setup_grid_aw<R, NP, 16>(p);
+template <int NP>
+static int setup_grid_np(gb_plan *p) {
+  return group_lanes(p->g.W) == 8 ? setup_grid_aw<NP, 8>(p) : setup_grid_aw<NP, 16>(p);
 }
 
 int setup_grid_kernels(gb_plan *p) {
-  if (p->precision == GB_FP64) {
-    switch (p->g.NP) {
-      case 1: return setup_grid_impl<double, 1>(p);
-      case 2: return setup_grid_impl<double, 2>(p);
-      default: return setup_grid_impl<double, 4>(p);
-    }
-  }
   switch (p->g.NP) {
-    case 1: return setup_grid_impl<float, 1>(p);
-    case 2: return setup_grid_impl<float, 2>(p);
-    default: return setup_grid_impl<float, 4>(p);
+    case 1: return setup_grid_np<1>(p);
+    case 2: return setup_grid_np<2>(p);
+    default: return setup_grid_np<4>(p);
   }
 }
 

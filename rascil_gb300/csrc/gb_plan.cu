@@ -252,6 +252,9 @@ static int plan_geometry_sigma(const gb_plan_params *p, double w_lo, double w_hi
   }
   g.T = T;
   g.S = S;
+  // FP64 form: short chunks, so that a chunk's cached kernel values leave room
+  // for several CTAs per SM (k_grid64)
+  g.chunk = p->precision == GB_FP64 ? kChunkItems64 : kChunkItems;
   g.ntu = (g.ngx + T - 1) / T;
   g.ntv = (g.ngy + T - 1) / T;
   g.nslabs = (g.nplanes + S - 1) / S;
@@ -506,26 +509,26 @@ __global__ void k_scatter(const Geom g, const double *__restrict__ uvw,
 
 // offsets[] is over sort keys (S per bucket): bucket b's items are
 // [offsets[b S], offsets[(b + 1) S]).
-__global__ void k_chunk_counts(const uint32_t *__restrict__ offsets, int S, int64_t nbuckets,
-                               uint32_t *__restrict__ ccounts) {
+__global__ void k_chunk_counts(const uint32_t *__restrict__ offsets, int S, uint32_t size,
+                               int64_t nbuckets, uint32_t *__restrict__ ccounts) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < nbuckets; b += stride) {
     const uint32_t n = offsets[(b + 1) * S] - offsets[b * S];
-    ccounts[b] = (n + kChunkItems - 1) / kChunkItems;
+    ccounts[b] = (n + size - 1) / size;
   }
 }
 
-__global__ void k_emit_chunks(const uint32_t *__restrict__ offsets, int S,
+__global__ void k_emit_chunks(const uint32_t *__restrict__ offsets, int S, uint32_t size,
                               const uint32_t *__restrict__ chunk_off, int64_t nbuckets,
                               Chunk *__restrict__ chunks) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < nbuckets; b += stride) {
     const uint32_t lo = offsets[b * S], hi = offsets[(b + 1) * S];
     uint32_t c = chunk_off[b];
-    for (uint32_t s = lo; s < hi; s += kChunkItems, ++c) {
+    for (uint32_t s = lo; s < hi; s += size, ++c) {
       Chunk ch;
       ch.begin = s;
-      ch.end = min(hi, s + (uint32_t)kChunkItems);
+      ch.end = min(hi, s + size);
       ch.bucket = (uint32_t)b;
       ch.pad = 0;
       chunks[c] = ch;
@@ -835,7 +838,7 @@ static int layout_workspace(gb_plan *p) {
   const size_t item_bytes = p->precision == GB_FP64 ? sizeof(ItemD) : sizeof(ItemF);
   const size_t cb = cplx_bytes(p->precision), rb = real_bytes(p->precision);
   const int64_t nb1 = g.nbuckets + 1;
-  p->max_chunks = (size_t)g.nitems / kChunkItems +
+  p->max_chunks = (size_t)g.nitems / g.chunk +
                   (size_t)std::min<int64_t>(g.nbuckets, (int64_t)g.nitems) + 1;
   p->nbatches = (g.nplanes + g.B - 1) / g.B;
   size_t off = 0;
@@ -949,12 +952,12 @@ static int run_bind(gb_plan *p, cudaStream_t s) {
     GB_LAUNCH_CHECK("k_scatter");
   }
   {
-    ProfScope ps(kProfChunks, s, 20.0 * (double)(nb + 1) + 16.0 * ni / kChunkItems);
-    k_chunk_counts<<<bucket_blocks, kThreads, 0, s>>>(offsets, g.S, nb, ccounts);
+    ProfScope ps(kProfChunks, s, 20.0 * (double)(nb + 1) + 16.0 * ni / g.chunk);
+    k_chunk_counts<<<bucket_blocks, kThreads, 0, s>>>(offsets, g.S, g.chunk, nb, ccounts);
     GB_LAUNCH_CHECK("k_chunk_counts");
     rc = scan_exclusive(ccounts, chunk_off, nb, stmp, s);
     if (rc) return rc;
-    k_emit_chunks<<<bucket_blocks, kThreads, 0, s>>>(offsets, g.S, chunk_off, nb, chunks);
+    k_emit_chunks<<<bucket_blocks, kThreads, 0, s>>>(offsets, g.S, g.chunk, chunk_off, nb, chunks);
     GB_LAUNCH_CHECK("k_emit_chunks");
   }
   // first item of every slab, to the host: only the profiler's byte counts

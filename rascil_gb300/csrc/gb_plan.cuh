@@ -129,6 +129,14 @@ int run_dirty2ms(gb_plan *p, const void *dirty, int layout, const void *wgt,
                  const PolMat &pm, int npv, void *vis, cudaStream_t s);
 int setup_tile_kernels(gb_plan *p);
 
+// FP64 tile kernels (gb_fp64.cu): gridding / degridding of planes [b0, b0 + nb)
+// fed from the batch's work counter; shared-memory opt-ins and grid sizes.
+int launch_grid64(gb_plan *p, int b0, int nb, const void *cvis, void *grid, uint32_t *counter,
+                  cudaStream_t s);
+int launch_degrid64(gb_plan *p, int b0, int nb, const void *grid, const void *wgt,
+                    const PolMat &pm, int npv, void *vis, uint32_t *counter, cudaStream_t s);
+int setup_tile_kernels64(gb_plan *p);
+
 // The same drivers in steps, for a batch of plans that interleaves them
 // (gb_batch.cu).  Invert: begin, then per w-plane batch bi zero -> grid ->
 // transform, then end.  Predict: begin, then per batch transform -> degrid.
