@@ -57,8 +57,8 @@ typedef enum { GB_FP32 = 0, GB_FP64 = 1 } gb_precision;
  * from 256 to 32768, twice the image height, even column offset), else
  * GB_FFT_CUFFT_2D.  GB_FFT_COLUMNS: the library's own column kernels,
  * pruned to the image's columns and fused with the w-screen, with its own
- * row kernels for grid widths 4096, 8192 and 16384 (else batched 1-D cuFFT
- * rows); asking for it where it does not apply is GB_ERR_INVALID_ARG.
+ * row kernels for power-of-two grid widths from 512 to 16384 (else batched
+ * 1-D cuFFT rows); asking for it where it does not apply is GB_ERR_INVALID_ARG.
  * GB_FFT_CUFFT_2D: batched 2-D cuFFT plans plus separate screen passes. */
 typedef enum { GB_FFT_AUTO = 0, GB_FFT_CUFFT_2D = 1, GB_FFT_COLUMNS = 2 } gb_fft_mode;
 
@@ -113,8 +113,9 @@ typedef struct {
   int64_t nitems, nbuckets, workspace_bytes;
   int32_t fft_mode;    /* the gb_fft_mode in use (never GB_FFT_AUTO)           */
   int32_t own_rows;    /* 1: GB_FFT_COLUMNS with the library's row transforms
-                          (grid width 4096, 8192 or 16384: no cuFFT plan, rows
-                          without visibilities skipped); 0: cuFFT rows      */
+                          (grid width a power of two from 512 to 16384: no
+                          cuFFT plan, cells without visibilities skipped);
+                          0: cuFFT rows                                     */
 } gb_plan_info;
 
 typedef struct gb_plan gb_plan;

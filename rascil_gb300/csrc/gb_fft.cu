@@ -1,7 +1,7 @@
 // Fused, pruned column transforms of the FP32 form.
 //
-// A w-plane's 2-D transform is done as row transforms (batched 1-D cuFFT
-// over contiguous rows) plus column transforms written here.  Column mode
+// A w-plane's 2-D transform is done as row transforms (gb_rows.cu, or batched
+// 1-D cuFFT for other widths) plus column transforms written here.  Column mode
 // applies when the grid height is a power of two and exactly twice the
 // image height (sigma = 2), so the image occupies the middle half of every
 // column (checkerboarded grids) and only the image's nx columns need
@@ -44,6 +44,7 @@
 #include <mutex>
 
 #include "gb_async.cuh"
+#include "gb_dft.cuh"
 #include "gb_fft.cuh"
 
 namespace gb {
@@ -58,20 +59,6 @@ struct ColShape {
   static_assert(M % T == 0 && M % 4 == 0 && T % 4 == 0, "column split");
 };
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ float2 cmulc(float2 a, float c, float s) {
-  return make_float2(a.x * c - a.y * s, a.x * s + a.y * c);
-}
-__device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-// a * (s i)
-template <int S> __device__ __forceinline__ float2 mul_si(float2 a) {
-  return S > 0 ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
-}
-
 // In-register L-point DFTs in natural order, z_q = sum_p a_p exp(s 2 pi i p q / L).
 template <int S> __device__ __forceinline__ void dft4(float2 *a) {
   const float2 s02 = cadd(a[0], a[2]), d02 = csub(a[0], a[2]);
@@ -81,10 +68,6 @@ template <int S> __device__ __forceinline__ void dft4(float2 *a) {
   a[1] = cadd(d02, d13);
   a[3] = csub(d02, d13);
 }
-
-constexpr float kR2 = 0.70710678118654752f;  // cos(pi/4)
-constexpr float kC8 = 0.92387953251128674f;  // cos(pi/8)
-constexpr float kS8 = 0.38268343236508977f;  // sin(pi/8)
 
 template <int S> __device__ __forceinline__ void dft8(float2 *a) {
   float2 e[4] = {a[0], a[2], a[4], a[6]};
@@ -131,10 +114,6 @@ template <int S> __device__ __forceinline__ void dft16(float2 *a) {
     for (int k2 = 0; k2 < 4; ++k2) a[k1 + 4 * k2] = b[k2];
   }
 }
-
-// cos / sin(2 pi k / 32), k < 16
-__device__ __constant__ float kCos32[16] = {1.0f, 0.98078528040323043f, 0.92387953251128674f, 0.83146961230254524f, 0.70710678118654757f, 0.55557023301960229f, 0.38268343236508984f, 0.19509032201612833f, 0.0f, -0.19509032201612819f, -0.38268343236508973f, -0.55557023301960196f, -0.70710678118654746f, -0.83146961230254535f, -0.92387953251128674f, -0.98078528040323043f};
-__device__ __constant__ float kSin32[16] = {0.0f, 0.19509032201612825f, 0.38268343236508978f, 0.55557023301960218f, 0.70710678118654746f, 0.83146961230254524f, 0.92387953251128674f, 0.98078528040323043f, 1.0f, 0.98078528040323043f, 0.92387953251128674f, 0.83146961230254546f, 0.70710678118654757f, 0.55557023301960218f, 0.38268343236508989f, 0.19509032201612861f};
 
 // 32 = 2 x 16: X[k] = E[k] + w^k O[k], X[k + 16] = E[k] - w^k O[k].
 template <int S> __device__ __forceinline__ void dft32(float2 *a) {
@@ -490,208 +469,6 @@ __global__ void __launch_bounds__(ColShape<N2>::THREADS, N2 >= 256 ? 1 : 3)
 }
 
 // ----------------------------------------------------------------------
-// Row transforms (both forms of the pass over contiguous rows), one CTA
-// per row with the whole row in shared memory.  N = R1 R2 R3 by two nested
-// four-step splits (all in registers, two shared-memory exchanges):
-//   pass 1  unit t < R2 R3 holds x[t + R2 R3 m], m < R1: R1-point DFT,
-//           times w_N^(t k1);
-//   pass 2  unit (k1, s), s < R3, holds the pass-1 outputs k1 of units
-//           s + R3 m': R2-point DFT, times w_(R2 R3)^(s k1');
-//   pass 3  unit (k1, k1') holds the pass-2 outputs k1' of units (k1, s):
-//           R3-point DFT, giving X[k1 + R1 k1' + R1 R2 k2'].
-// Input columns outside [in_lo, in_hi) are taken as zero (predict: only the
-// image columns hold data) and only outputs in [out_lo, out_hi) are stored
-// (invert: only the image columns are needed).  The first N/2 input cells of
-// the next row stream into a shared-memory stage by one bulk copy (mbarrier
-// completion) while the current row's passes 2 and 3 and its stores run;
-// the rest of the input (invert's second half) is loaded directly, its next
-// row prefetched into L2.  A staging wait past its limit records
-// kErrTmaTimeout in *status, waits once more (bounded) for the copy in
-// flight and returns.  Rows whose (plane, row
-// tile) is empty in the occupancy mask are skipped: an invert row there is
-// zero (nothing gridded), a predict row there is never degridded.
-template <int N> struct RowShape;
-template <> struct RowShape<16384> {
-  static constexpr int R1 = 32, R2 = 32, R3 = 16, THREADS = 512, MINB = 1;
-};
-template <> struct RowShape<8192> {
-  static constexpr int R1 = 32, R2 = 16, R3 = 16, THREADS = 256, MINB = 2;
-};
-template <> struct RowShape<4096> {
-  static constexpr int R1 = 32, R2 = 16, R3 = 8, THREADS = 128, MINB = 4;
-};
-
-struct RowArgs {
-  float2 *grid;              // batch buffer: rows of ngx cells
-  const uint8_t *mask;       // [nplanes][ntv] occupancy, or null
-  const float2 *twx;         // exp(+2 pi i m / ngx), m < ngx
-  int64_t nrows;             // nb NP ngy rows in this batch
-  int ngy, NP, b0, T, ntv;
-  int perm_s1, perm_s2;      // predict rows: logical row of physical r, or -1
-  int in_lo, in_hi, out_lo, out_hi;
-  uint32_t *status;          // kErrTmaTimeout when a staging wait runs past its limit
-};
-
-template <int N, int S>
-__global__ void __launch_bounds__(RowShape<N>::THREADS, RowShape<N>::MINB)
-    k_rows(const RowArgs ra) {
-  using RS = RowShape<N>;
-  constexpr int R1 = RS::R1, R2 = RS::R2, R3 = RS::R3, TH = RS::THREADS;
-  constexpr int TN = R2 * R3;  // pass-1 units
-  constexpr int NA = N / 128;  // two-level twiddle table: w^m = A[m >> 7] B[m & 127]
-  static_assert(TN == TH, "one pass-1 unit per thread");
-  constexpr int NH = N / 2;  // staged input cells per row
-  extern __shared__ __align__(16) float2 smem[];
-  float2 *ex = smem;                        // exchange: max(R1 (TN + 1), N) cells
-  float2 *ta = smem + R1 * (TN + 1);        // [NA]
-  float2 *tb = ta + NA;                     // [128]
-  float2 *t2 = tb + 128;                    // [TN]: w_TN^m = w_N^(R1 m)
-  float2 *stg = t2 + TN;                    // [NH]: the next row's first input cells
-  __shared__ __align__(8) uint64_t s_bar;
-  __shared__ int s_abort;
-  // staged: input elements m in [m_lo, m_hi) of pass 1 (col = t + TN m), so
-  // whole multiples of TN cells (always so for the image-column ranges)
-  const int st_lo = ra.in_lo;
-  const int st_n = (st_lo % TN == 0 && ra.in_hi % TN == 0) ? min(ra.in_hi - ra.in_lo, NH) : 0;
-  const int m_lo = st_lo / TN, m_hi = (st_lo + st_n) / TN;
-  const unsigned st_bytes = (unsigned)st_n * (unsigned)sizeof(float2);
-  if (threadIdx.x == 0) {
-    mbar_init(&s_bar, 1);
-    s_abort = 0;
-    fence_mbarrier_init();
-  }
-  for (int i = threadIdx.x; i < NA + 128; i += TH) {
-    const float2 w = ra.twx[i < NA ? i * 128 : i - NA];
-    (i < NA ? ta[i] : tb[i - NA]) = S > 0 ? w : conjf2(w);
-  }
-  for (int i = threadIdx.x; i < TN; i += TH) {
-    const float2 w = ra.twx[i * R1];
-    t2[i] = S > 0 ? w : conjf2(w);
-  }
-  __syncthreads();
-  auto tw = [&](int m) { return cmul(ta[m >> 7], tb[m & 127]); };
-  auto used = [&](int64_t row) {
-    if (!ra.mask) return true;
-    const int sp = (int)(row / ra.ngy), r = (int)(row - (int64_t)sp * ra.ngy);
-    const int q = ra.perm_s1 < 0 ? r
-                                 : (r >> ra.perm_s2) + ((r & ((1 << ra.perm_s2) - 1)) << ra.perm_s1);
-    return ra.mask[(int64_t)(ra.b0 + sp / ra.NP) * ra.ntv + q / ra.T] != 0;
-  };
-  // the next used row this CTA will transform, prefetched into L2 while
-  // this one is transformed (one CTA per SM leaves no other row in flight)
-  auto next_used = [&](int64_t row) {
-    for (row += gridDim.x; row < ra.nrows && !used(row); row += gridDim.x) {
-    }
-    return row;
-  };
-  // the unstaged input of a row, prefetched into L2
-  auto prefetch_row = [&](int64_t row) {
-    if (threadIdx.x == 0 && row < ra.nrows && st_lo + st_n < ra.in_hi)
-      prefetch_l2(ra.grid + row * N + st_lo + st_n,
-                  (unsigned)((ra.in_hi - st_lo - st_n) * sizeof(float2)));
-  };
-  // the staged input of a row (thread 0; the stage's earlier generic reads
-  // are ordered before the copy by the barrier and the proxy fence)
-  auto stage_row = [&](int64_t row) {
-    fence_proxy_async();
-    mbar_expect_tx(&s_bar, st_bytes);
-    bulk_load(stg, ra.grid + row * N + st_lo, st_bytes, &s_bar);
-  };
-  const int t = threadIdx.x;
-  int64_t row = blockIdx.x;
-  if (row < ra.nrows && !used(row)) row = next_used(row);
-  __syncthreads();  // the barrier's initialisation before any wait on it
-  if (threadIdx.x == 0 && row < ra.nrows && st_n) stage_row(row);
-  prefetch_row(row);
-  unsigned phase = 0;
-  for (; row < ra.nrows;) {
-    const int64_t next = next_used(row);
-    prefetch_row(next);
-    float2 *rp = ra.grid + row * N;
-    if (st_n) {
-      if (!mbar_wait(&s_bar, phase)) s_abort = 1;
-      phase ^= 1u;
-    }
-    // pass 1
-    float2 x[R1];
-#pragma unroll
-    for (int m = 0; m < R1; ++m) {
-      const int col = t + TN * m;
-      x[m] = (m >= m_lo && m < m_hi)
-                 ? stg[t + TN * (m - m_lo)]
-                 : ((col >= ra.in_lo && col < ra.in_hi) ? rp[col] : make_float2(0.f, 0.f));
-    }
-    dft<R1, S>(x);
-    {
-      // w^(t k1), k1 < 32, as w^(t (k1 & 7)) w^(8 t (k1 >> 3)): powers of w^t
-      // by multiplication (at most 7 roundings) times three table values
-      float2 pw[8], qw[4];
-      pw[0] = make_float2(1.f, 0.f);
-      pw[1] = tw(t);
-#pragma unroll
-      for (int j = 2; j < 8; ++j) pw[j] = cmul(pw[j - 1], pw[1]);
-      qw[0] = pw[0];
-#pragma unroll
-      for (int i = 1; i < R1 / 8; ++i) qw[i] = tw((8 * t * i) & (N - 1));
-      static_assert(R1 == 32, "pass-1 twiddle split");
-#pragma unroll
-      for (int k1 = 0; k1 < R1; ++k1) {
-        float2 v = x[k1];
-        if (k1 & 7) v = cmul(v, pw[k1 & 7]);
-        if (k1 >> 3) v = cmul(v, qw[k1 >> 3]);
-        ex[k1 * (TN + 1) + t] = v;
-      }
-    }
-    __syncthreads();  // pass-1 exchange written; the stage read by every thread
-    if (s_abort) {
-      if (threadIdx.x == 0) {
-        atomicOr(ra.status, kErrTmaTimeout);
-        mbar_wait(&s_bar, phase ^ 1u);  // (bounded) the copy still in flight
-      }
-      return;
-    }
-    if (threadIdx.x == 0 && next < ra.nrows && st_n) stage_row(next);
-    // pass 2: units u = k1 + R1 s
-    constexpr int U2 = R1 * R3 / TH;
-    float2 y[U2][R2];
-#pragma unroll
-    for (int i = 0; i < U2; ++i) {
-      const int u = t + TH * i, k1 = u % R1, s = u / R1;
-#pragma unroll
-      for (int m = 0; m < R2; ++m) y[i][m] = ex[k1 * (TN + 1) + s + R3 * m];
-      dft<R2, S>(y[i]);
-#pragma unroll
-      for (int k = 1; k < R2; ++k) y[i][k] = cmul(y[i][k], t2[s * k]);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < U2; ++i) {
-      const int u = t + TH * i, k1 = u % R1, s = u / R1;
-#pragma unroll
-      for (int k = 0; k < R2; ++k) ex[(k * R3 + s) * R1 + k1] = y[i][k];
-    }
-    __syncthreads();
-    // pass 3: units u = k1 + R1 k1'
-    constexpr int U3 = R1 * R2 / TH;
-#pragma unroll
-    for (int i = 0; i < U3; ++i) {
-      const int u = t + TH * i, k1 = u % R1, kp = u / R1;
-      float2 z[R3];
-#pragma unroll
-      for (int s = 0; s < R3; ++s) z[s] = ex[(kp * R3 + s) * R1 + k1];
-      dft<R3, S>(z);
-#pragma unroll
-      for (int k2 = 0; k2 < R3; ++k2) {
-        const int o = k1 + R1 * kp + R1 * R2 * k2;
-        if (o >= ra.out_lo && o < ra.out_hi) rp[o] = z[k2];
-      }
-    }
-    __syncthreads();  // exchange slots free for the next row
-    row = next;
-  }
-}
-
-// ----------------------------------------------------------------------
 // host side
 
 static int ilog2(int n) {
@@ -826,7 +603,7 @@ static int cols_invert_np(gb_plan *p, float2 *grid, int b0, int nb, float *acc, 
                           cudaStream_t s) {
   const Geom &g = p->g;
   ColGeom cg = col_geom(g);
-  cg.mask = p->at<uint8_t>(p->off_rowmask);
+  cg.mask = p->at<uint32_t>(p->off_rowmask);
   cg.b0 = b0;
   const unsigned tiles = (unsigned)((g.nx + kCW - 1) / kCW);
   const float2 *twn = p->at<float2>(p->off_twn);
@@ -877,7 +654,7 @@ static int cols_predict_np(gb_plan *p, const float *img, int b0, int nb, float2 
                            cudaStream_t s) {
   const Geom &g = p->g;
   ColGeom cg = col_geom(g);
-  cg.mask = p->at<uint8_t>(p->off_rowmask);
+  cg.mask = p->at<uint32_t>(p->off_rowmask);
   cg.b0 = b0;
   const unsigned tiles = (unsigned)((g.nx + kCW - 1) / kCW);
   const float2 *twn = p->at<float2>(p->off_twn);
@@ -924,108 +701,6 @@ static int cols_predict_np(gb_plan *p, const float *img, int b0, int nb, float2 
     if (left) GB_CUDA(cudaMemset2DAsync(grid, pitch, 0, left, rows, s));
     if (right) GB_CUDA(cudaMemset2DAsync(grid + cg.ox + g.nx, pitch, 0, right, rows, s));
   }
-  return GB_OK;
-}
-
-// Zero the used rows (mask) of nrows = nb NP ngy rows of ngx cells.
-__global__ void k_zero_rows(float2 *__restrict__ grid, const uint8_t *__restrict__ mask,
-                            int64_t nrows, int ngx, int ngy, int NP, int b0, int T, int ntv) {
-  const int n4 = ngx / 2;  // float4 per row (ngx even)
-  for (int64_t row = blockIdx.x; row < nrows; row += gridDim.x) {
-    const int sp = (int)(row / ngy), r = (int)(row - (int64_t)sp * ngy);
-    if (!mask[(int64_t)(b0 + sp / NP) * ntv + r / T]) continue;
-    float4 *dst = reinterpret_cast<float4 *>(grid + row * ngx);
-    for (int i = threadIdx.x; i < n4; i += blockDim.x) dst[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-}
-
-int run_zero_rows(gb_plan *p, void *grid, int b0, int nb, cudaStream_t s) {
-  const Geom &g = p->g;
-  const int64_t nrows = (int64_t)nb * g.NP * g.ngy;
-  const unsigned blocks = (unsigned)std::min<int64_t>(nrows, (int64_t)p->num_sms * 8);
-  k_zero_rows<<<blocks, kThreads, 0, s>>>(reinterpret_cast<float2 *>(grid),
-                                          p->at<uint8_t>(p->off_rowmask), nrows, g.ngx, g.ngy,
-                                          g.NP, b0, g.T, g.ntv);
-  GB_LAUNCH_CHECK("k_zero_rows");
-  return GB_OK;
-}
-
-bool row_kernel_fits(int n) { return n == 4096 || n == 8192 || n == 16384; }
-
-template <int N> constexpr size_t rows_smem() {
-  using RS = RowShape<N>;
-  return sizeof(float2) *
-         ((size_t)RS::R1 * (RS::R2 * RS::R3 + 1) + N / 128 + 128 + RS::R2 * RS::R3 + N / 2);
-}
-
-template <int N, int S> static int rows_occupancy(int *per_sm) {
-  GB_CUDA(cudaFuncSetAttribute(k_rows<N, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)rows_smem<N>()));
-  GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_rows<N, S>,
-                                                        RowShape<N>::THREADS, rows_smem<N>()));
-  return GB_OK;
-}
-
-int setup_row_kernels(gb_plan *p) {
-  if (!p->row_fft) return GB_OK;
-  int a = 0, b = 0, rc;
-  switch (p->g.ngx) {
-    case 4096: rc = rows_occupancy<4096, 1>(&a); if (!rc) rc = rows_occupancy<4096, -1>(&b); break;
-    case 8192: rc = rows_occupancy<8192, 1>(&a); if (!rc) rc = rows_occupancy<8192, -1>(&b); break;
-    default: rc = rows_occupancy<16384, 1>(&a); if (!rc) rc = rows_occupancy<16384, -1>(&b); break;
-  }
-  if (rc) return rc;
-  if (std::min(a, b) < 1) {
-    set_error("k_rows cannot launch for rows of %d cells", p->g.ngx);
-    return GB_ERR_INVALID_ARG;
-  }
-  p->row_blocks = std::min(a, b) * p->num_sms;
-  return GB_OK;
-}
-
-int run_rows(gb_plan *p, void *grid, int b0, int nb, int dir, cudaStream_t s) {
-  const Geom &g = p->g;
-  const ColGeom cg = col_geom(g);
-  RowArgs ra;
-  ra.grid = reinterpret_cast<float2 *>(grid);
-  ra.mask = p->at<uint8_t>(p->off_rowmask);
-  ra.twx = p->at<float2>(p->off_twx);
-  ra.nrows = (int64_t)nb * g.NP * g.ngy;
-  ra.ngy = g.ngy;
-  ra.NP = g.NP;
-  ra.b0 = b0;
-  ra.T = g.T;
-  ra.ntv = g.ntv;
-  ra.status = p->status_word();
-  if (dir > 0) {  // invert: full rows in, image columns out
-    ra.perm_s1 = -1;
-    ra.perm_s2 = 0;
-    ra.in_lo = 0;
-    ra.in_hi = g.ngx;
-    ra.out_lo = cg.ox;
-    ra.out_hi = cg.ox + g.nx;
-  } else {  // predict: image columns in (rest taken as zero), full rows out
-    const RowPerm rp = row_perm(p);
-    ra.perm_s1 = rp.s1;
-    ra.perm_s2 = rp.s2;
-    ra.in_lo = cg.ox;
-    ra.in_hi = cg.ox + g.nx;
-    ra.out_lo = 0;
-    ra.out_hi = g.ngx;
-  }
-  const unsigned blocks = (unsigned)std::min<int64_t>(p->row_blocks, ra.nrows);
-#define GB_ROWS(N)                                                                        \
-  if (dir > 0)                                                                            \
-    k_rows<N, 1><<<blocks, RowShape<N>::THREADS, rows_smem<N>(), s>>>(ra);                \
-  else                                                                                    \
-    k_rows<N, -1><<<blocks, RowShape<N>::THREADS, rows_smem<N>(), s>>>(ra);
-  switch (g.ngx) {
-    case 4096: GB_ROWS(4096) break;
-    case 8192: GB_ROWS(8192) break;
-    default: GB_ROWS(16384) break;
-  }
-#undef GB_ROWS
-  GB_LAUNCH_CHECK("k_rows");
   return GB_OK;
 }
 

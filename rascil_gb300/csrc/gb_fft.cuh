@@ -1,5 +1,5 @@
-// Column transforms of the FP32 form (gb_fft.cu) and the row order they
-// leave in predict grids.
+// Column and row transforms of the FP32 form (gb_fft.cu, gb_rows.cu) and the
+// row order that the columns leave in predict grids.
 #pragma once
 
 #include "gb_plan.cuh"
@@ -16,10 +16,10 @@ struct ColGeom {
   int64_t plane;   // ngx * ngy
   int ngx;
   // (plane, row tile) occupancy: invert step A takes rows outside it as zero
-  const uint8_t *mask;
+  const uint32_t *mask;
   int b0, NP, T, ntv;
   __device__ __forceinline__ bool row_used(int pp, int q) const {
-    return !mask || mask[(int64_t)(b0 + pp / NP) * ntv + q / T];
+    return !mask || mask[(int64_t)(b0 + pp / NP) * ntv + q / T] != 0;
   }
 };
 
@@ -31,17 +31,18 @@ RowPerm row_perm(const gb_plan *p);
 
 // Shared-memory opt-ins of the column kernels (plan creation).
 int setup_col_kernels(gb_plan *p);
-// Zero the rows of the batch buffer that the occupancy mask marks as used
-// (the others are never read); column mode's replacement for a memset.
+// Zero what the gridder writes in the batch buffer: the occupied bins of the
+// mask, or with cuFFT rows the whole rows of occupied tiles (the others are
+// never read); column mode's replacement for a memset.
 int run_zero_rows(gb_plan *p, void *grid, int b0, int nb, cudaStream_t s);
-// Row lengths with a k_rows instantiation (4096, 8192, 16384).
-bool row_kernel_fits(int n);
+// Row lengths with a k_rows instantiation (512 to 16384, powers of two) for an
+// image of nx columns (the middle half of the row at most).
+bool row_kernel_fits(int n, int nx);
 // Occupancy / opt-ins of the row kernels (plan creation).
 int setup_row_kernels(gb_plan *p);
-// Row transforms of nb planes x NP pols of the batch buffer: dir > 0
-// invert (e^{+}, full rows in, image columns out), dir < 0 predict (e^{-},
-// image columns in, full rows out); rows empty in the occupancy mask are
-// skipped.
+// Row transforms of nb planes x NP pols of the batch buffer: dir > 0 invert
+// (e^{+}, occupied bins in, image columns out), dir < 0 predict (e^{-}, image
+// columns in, occupied bins out); rows without occupied bins are skipped.
 int run_rows(gb_plan *p, void *grid, int b0, int nb, int dir, cudaStream_t s);
 // Invert: step A in place, then step B fused with the w-screen and the
 // image accumulation (first != 0 starts acc from zero).

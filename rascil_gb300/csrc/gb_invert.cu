@@ -634,8 +634,9 @@ static int inv_zero_impl(gb_plan *p, int bi, cudaStream_t s) {
   C *grid = reinterpret_cast<C *>(p->ws + p->off_temp + p->c_grid);
   const int b0 = bi * g.B, nb = std::min(g.B, g.nplanes - b0);
   const double gbytes = (double)sizeof(C) * nb * NP * (double)g.ngx * g.ngy;
-  if (p->col_fft) {  // only rows the gridder writes; column step A skips the rest
-    ProfScope ps(kProfGridZero, s, p->used_rows(b0, nb) * gbytes);
+  if (p->col_fft) {  // only what the gridder writes; the transforms skip the rest
+    ProfScope ps(kProfGridZero, s,
+                 (p->row_fft ? p->used_cells(b0, nb) : p->used_rows(b0, nb)) * gbytes);
     return run_zero_rows(p, grid, b0, nb, s);
   }
   ProfScope ps(kProfGridZero, s, gbytes);
@@ -702,8 +703,9 @@ static int inv_transform_impl(gb_plan *p, int bi, cudaStream_t s) {
   const int64_t npix = (int64_t)g.nx * g.ny;
   int rc;
   if (p->row_fft) {
-    // used rows: read, image half written
-    ProfScope ps(kProfRowsInv, s, 1.5 * p->used_rows(b0, nb) * gbytes);
+    // occupied bins read, image half of the used rows written
+    ProfScope ps(kProfRowsInv, s,
+                 (p->used_cells(b0, nb) + 0.5 * p->used_rows(b0, nb)) * gbytes);
     rc = run_rows(p, grid, b0, nb, 1, s);
   } else {
     ProfScope ps(kProfFftInv, s, 2.0 * gbytes);

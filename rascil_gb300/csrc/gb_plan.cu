@@ -578,23 +578,39 @@ __global__ void k_corr_image(const Geom g, const double *__restrict__ cu,
   }
 }
 
-// Occupancy of (w-plane, row tile): a chunk's items reach planes
-// [slab S, slab S + S + W - 1) and rows [tv T, tv T + T + W - 1) (mod ngy).
-__global__ void k_row_mask(const Geom g, const Chunk *__restrict__ chunks,
-                           const uint32_t *__restrict__ chunk_off, uint8_t *__restrict__ mask) {
+// Occupancy mask: per (w-plane, row tile) a word whose bit b marks cells
+// [b bw, (b + 1) bw) of the tile's rows, bw = ceil(ngx / 32).  A chunk's items (in
+// order of first w-plane) reach planes from its first item's first to its
+// last item's last, rows [tv T, tv T + T + W - 1) and columns [tu T, tu T + T + W - 1)
+// (mod the grid).
+__global__ void k_row_mask(const Geom g, const ItemF *__restrict__ items,
+                           const Chunk *__restrict__ chunks,
+                           const uint32_t *__restrict__ chunk_off, uint32_t *__restrict__ mask) {
   const uint32_t nch = chunk_off[g.nbuckets];
-  const int ntiles = g.ntu * g.ntv;
+  const int ntiles = g.ntu * g.ntv, wk = g.do_w ? g.W : 1;
+  const int bw = (g.ngx + 31) / 32;
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nch; c += gridDim.x * blockDim.x) {
-    const uint32_t bucket = chunks[c].bucket;
-    const int slab = (int)(bucket / (uint32_t)ntiles);
-    const int tv = (int)(bucket - (uint32_t)slab * ntiles) / g.ntu;
-    const int k_lo = slab * g.S, k_hi = min(k_lo + g.S + g.W - 1, g.nplanes);
+    const Chunk ch = chunks[c];
+    const int slab = (int)(ch.bucket / (uint32_t)ntiles);
+    const int tile = (int)(ch.bucket - (uint32_t)slab * ntiles);
+    const int tv = tile / g.ntu, tu = tile - tv * g.ntu;
+    uint32_t bits = 0;
+    const int c_hi = tu * g.T + g.T + g.W - 2;  // inclusive
+    for (int x = tu * g.T; x <= c_hi + bw - 1; x += bw) {
+      int xx = min(x, c_hi);
+      while (xx >= g.ngx) xx -= g.ngx;
+      bits |= 1u << (xx / bw);
+    }
+    const int k_lo = slab * g.S + (int)((items[ch.begin].loc >> 16) & 0xffu);
+    const int k_hi =
+        min(slab * g.S + (int)((items[ch.end - 1].loc >> 16) & 0xffu) + wk, g.nplanes);
     const int r_lo = tv * g.T, r_hi = tv * g.T + g.T + g.W - 2;  // inclusive
     for (int k = k_lo; k < k_hi; ++k) {
       for (int r = r_lo; r <= r_hi + g.T - 1; r += g.T) {
         int rr = min(r, r_hi);
         while (rr >= g.ngy) rr -= g.ngy;
-        mask[(int64_t)k * g.ntv + rr / g.T] = 1;
+        uint32_t *w = &mask[(int64_t)k * g.ntv + rr / g.T];
+        if ((*w & bits) != bits) atomicOr(w, bits);
       }
     }
   }
@@ -829,7 +845,7 @@ static int choose_fft_mode(gb_plan *p) {
       set_error("unknown fft_mode %d", p->params.fft_mode);
       return GB_ERR_INVALID_ARG;
   }
-  p->row_fft = p->col_fft && row_kernel_fits(p->g.ngx);
+  p->row_fft = p->col_fft && row_kernel_fits(p->g.ngx, p->g.nx);
   return GB_OK;
 }
 
@@ -859,7 +875,7 @@ static int layout_workspace(gb_plan *p) {
   p->off_twx = off;
   off = align_up(off + (p->row_fft ? 8 * (size_t)g.ngx : 0));
   p->off_rowmask = off;
-  off = align_up(off + (p->col_fft ? (size_t)g.nplanes * g.ntv : 0));
+  off = align_up(off + (p->col_fft ? 4 * (size_t)g.nplanes * g.ntv : 0));
   p->off_tables = off;
   off = align_up(off + 8 * ((size_t)g.nx + g.ny + 2 * kMaxQuad));
   // shifted plans keep uvw and f/c: a PSF call rebuilds the unshifted factor
@@ -998,15 +1014,15 @@ static int run_bind(gb_plan *p, cudaStream_t s) {
     GB_LAUNCH_CHECK("k_twiddles");
   }
   if (p->col_fft) {
-    uint8_t *mask = p->at<uint8_t>(p->off_rowmask);
-    GB_CUDA(cudaMemsetAsync(mask, 0, (size_t)g.nplanes * g.ntv, s));
+    uint32_t *mask = p->at<uint32_t>(p->off_rowmask);
+    GB_CUDA(cudaMemsetAsync(mask, 0, 4 * (size_t)g.nplanes * g.ntv, s));
     const unsigned cb = (unsigned)std::min<int64_t>(
         ((int64_t)p->max_chunks + kThreads - 1) / kThreads, (int64_t)p->num_sms * 16);
-    k_row_mask<<<cb, kThreads, 0, s>>>(g, chunks, chunk_off, mask);
+    k_row_mask<<<cb, kThreads, 0, s>>>(g, p->at<ItemF>(p->off_items), chunks, chunk_off, mask);
     GB_LAUNCH_CHECK("k_row_mask");
     if (prof_on()) {  // host copy for the profiler's byte counts (costs a sync)
       p->mask_host.assign((size_t)g.nplanes * g.ntv, 0);
-      GB_CUDA(cudaMemcpyAsync(p->mask_host.data(), mask, p->mask_host.size(),
+      GB_CUDA(cudaMemcpyAsync(p->mask_host.data(), mask, 4 * p->mask_host.size(),
                               cudaMemcpyDeviceToHost, s));
       GB_CUDA(cudaStreamSynchronize(s));
     }

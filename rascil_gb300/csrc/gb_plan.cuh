@@ -39,8 +39,8 @@ struct gb_plan {
   // column mode (FP32): the plans above are 1-D row transforms and the
   // column transforms are the library's own kernels (gb_fft.cu)
   bool col_fft = false;
-  // column mode with rows of 4096 / 8192 / 16384 cells: the row transforms
-  // are k_rows too (no cuFFT plan), with a (plane, row tile) occupancy mask
+  // column mode with rows of 512 to 16384 cells (powers of two): the row
+  // transforms are k_rows (no cuFFT plan), which follow the occupancy mask
   bool row_fft = false;
   size_t off_rowmask = 0, off_twx = 0;
   int row_blocks = 0;
@@ -55,7 +55,7 @@ struct gb_plan {
   int num_sms = 0;
   int grid_blocks = 0, degrid_blocks = 0;  // persistent grid sizes
   std::vector<uint32_t> slab_items;        // host copy: first item of each slab (+ total)
-  std::vector<uint8_t> mask_host;          // host copy of the occupancy mask (profiling)
+  std::vector<uint32_t> mask_host;         // host copy of the occupancy mask (profiling)
   // profiling only: per w-plane, grid cells in the (plane, uv tile) pairs
   // some item reaches (tile cells plus the support halo spilling into
   // tiles nothing reaches), and items whose first plane is that plane
@@ -80,14 +80,20 @@ struct gb_plan {
     return n;
   }
 
-  // Fraction of the rows of planes [b0, b0 + nb) that visibilities reach
-  // (occupancy mask; 1 without one).  Profiling byte counts only.
-  double used_rows(int b0, int nb) const {
+  // Fraction of the rows of planes [b0, b0 + nb) that visibilities reach, and
+  // of their cells in occupied bins (occupancy mask; 1 without one).
+  // Profiling byte counts only.
+  double used_rows(int b0, int nb) const { return mask_fraction(b0, nb, 32); }
+  double used_cells(int b0, int nb) const { return mask_fraction(b0, nb, 1); }
+  double mask_fraction(int b0, int nb, int per_bin) const {
     if (mask_host.empty() || nb <= 0) return 1.0;
     int64_t used = 0;
     for (int k = b0; k < b0 + nb; ++k)
-      for (int t = 0; t < g.ntv; ++t) used += mask_host[(size_t)k * g.ntv + t];
-    return (double)used / ((double)nb * g.ntv);
+      for (int t = 0; t < g.ntv; ++t) {
+        const uint32_t w = mask_host[(size_t)k * g.ntv + t];
+        used += per_bin == 32 ? (w ? 32 : 0) : __builtin_popcount(w);
+      }
+    return (double)used / (32.0 * nb * g.ntv);
   }
 
   // items whose w-slab reaches planes [b0, b0 + nb)

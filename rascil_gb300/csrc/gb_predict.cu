@@ -516,8 +516,9 @@ static int pred_transform_impl(gb_plan *p, int bi, cudaStream_t s) {
     GB_LAUNCH_CHECK("k_screen_pad");
   }
   if (p->row_fft) {
-    // image half in, row out
-    ProfScope ps(kProfRowsFwd, s, 1.5 * p->used_rows(b0, nb) * gbytes);
+    // image half in, occupied bins out
+    ProfScope ps(kProfRowsFwd, s,
+                 (p->used_cells(b0, nb) + 0.5 * p->used_rows(b0, nb)) * gbytes);
     return run_rows(p, grid, b0, nb, -1, s);
   }
   ProfScope ps(kProfFftFwd, s, 2.0 * gbytes);
