@@ -458,8 +458,8 @@ int launch_degrid64(gb_plan *p, int b0, int nb, const void *grid, const void *wg
 template <int NP>
 static int setup_np(gb_plan *p) {
   const size_t smem = grid64_smem_bytes(p->g);
-  GB_CUDA(cudaFuncSetAttribute(k_grid64<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem));
+  const int rc = allow_shared_memory(k_grid64<NP>);
+  if (rc) return rc;
   int per_sm = 0;
   GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_grid64<NP>, kThreads, smem));
   if (per_sm < 1) {

@@ -886,7 +886,8 @@ int launch_grid_jobs(const GridJobs &jobs, int num_sms, uint32_t *counter, doubl
 #define GB_GJ(NPV, AWV)                                                                      \
   {                                                                                          \
     auto k = k_grid_jobs<NPV, AWV>;                                                          \
-    GB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+    const int rc = allow_shared_memory(k);                                                   \
+    if (rc) return rc;                                                                       \
     int per_sm = 0;                                                                          \
     GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem));      \
     if (per_sm < 1) {                                                                        \
@@ -942,7 +943,8 @@ template <int NP, int AW>
 static int setup_grid_aw(gb_plan *p) {
   const size_t smem = grid_smem_bytes(p);
   auto k = k_grid<NP, AW>;
-  GB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int rc = allow_shared_memory(k);
+  if (rc) return rc;
   int per_sm = 0;
   GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem));
   if (per_sm < 1) {

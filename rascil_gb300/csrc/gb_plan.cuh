@@ -154,6 +154,21 @@ int inv_end(gb_plan *p, void *dirty, int layout, cudaStream_t s);
 int pred_begin(gb_plan *p, const void *dirty, int layout, cudaStream_t s);
 int pred_transform(gb_plan *p, int bi, cudaStream_t s);
 
+// Let a kernel be launched with any dynamic shared memory the device grants a
+// block.  Never the size of one plan: the opt-in is per kernel, and a plan of
+// smaller tiles made later would lower it under the launches of a larger one.
+template <typename K> int allow_shared_memory(K kernel) {
+  int dev = 0, most = 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             most - (int)a.sharedSizeBytes);
+  return e == cudaSuccess ? (int)GB_OK : cuda_fail(e, "shared-memory opt-in");
+}
+
 // Polarisation matrix from a host array of nout x nin complex (re, im
 // interleaved; NULL = identity, which needs nout == nin).
 int make_polmat(const double *host, int nout, int nin, PolMat &pm);

@@ -79,3 +79,26 @@ def test_non_finite_values_reach_their_polarisation_only(bad):
     got = plan.ms2dirty(torch.from_numpy(c["ms"]).cuda(), layout="yx").cpu().numpy()
     assert not numpy.isfinite(got[1]).any()
     assert rel_rms(got[0], clean[0]) < 1e-14
+
+
+@pytest.mark.parametrize("precision,eps,kw", [
+    ("fp64", 8e-14, [{}, dict(support=4)]),
+    ("fp32", 1e-5, [dict(tile=48), dict(tile=4)]),
+])
+def test_plans_of_other_shared_memory_do_not_disturb_each_other(precision, eps, kw):
+    """A kernel's shared-memory opt-in belongs to the kernel: a plan that needs
+    little, made later, must not take it from one that needs more."""
+    import torch
+    from rascil_gb300 import wgridder
+    c = random_problem(seed=6, nrow=200, nchan=1, npix=64)
+    u = torch.from_numpy(c["uvw"]).cuda()
+    f = torch.from_numpy(c["freq"]).cuda()
+    ms = torch.from_numpy(c["ms"]).cuda()
+    plans = []
+    for extra in kw:
+        p = wgridder.Plan(u, f, 64, 64, c["pixsize"], c["pixsize"], eps, True, npol=1,
+                          precision=precision, sigma=2.0, **extra)
+        plans.append((p, p.ms2dirty(ms.to(p.complex_dtype), layout="yx").clone()))
+    for p, before in plans:
+        again = p.ms2dirty(ms.to(p.complex_dtype), layout="yx")
+        assert rel_rms(again.cpu().numpy(), before.cpu().numpy()) < 1e-6
