@@ -544,37 +544,54 @@ __global__ void k_slab_items(const uint32_t *__restrict__ offsets, int nslabs, i
 
 // Correction image [ny][nx]: 1/(phihat_u phihat_v) and, with w-stacking,
 // 1/(phihat_w(dw t') n).  phihat_w by Gauss-Legendre quadrature of the
-// (even) kernel on [0, W/2].
+// (even) kernel on [0, W/2], in the form's own precision (nodes rounded once on
+// the host: a conversion is an FP64-pipe instruction, 16 cycles a warp).  The
+// image is even in x and y about pixel n/2, so a thread forms the value of pixel
+// (ix, iy), ix <= nx/2, iy <= ny/2, and writes it to its mirrors too: a quarter of
+// the square roots, divisions and cosines.  8192^2 pixels: 13.8 ms with a
+// thread per pixel and FP64 nodes, 1.9 ms like this.
+template <typename R> struct QuadIn {
+  int n;
+  R x[kMaxQuad], w[kMaxQuad];
+};
 
 template <typename R>
 __global__ void k_corr_image(const Geom g, const double *__restrict__ cu,
-                             const double *__restrict__ cv, const Quad quad,
+                             const double *__restrict__ cv, const QuadIn<R> quad,
                              R *__restrict__ corr, double *__restrict__ tprime,
                              ulonglong2 *__restrict__ screen) {
-  const int64_t npix = (int64_t)g.nx * g.ny;
+  const int hx = g.nx / 2 + 1, hy = g.ny / 2 + 1;
+  const int64_t n = (int64_t)hx * hy;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < npix; i += stride) {
-    const int iy = (int)(i / g.nx), ix = (int)(i - (int64_t)iy * g.nx);
-    double f = cu[ix] * cv[iy];
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
+    const int iy = (int)(i / hx), ix = (int)(i - (int64_t)iy * hx);
+    double f = cu[ix] * cv[iy], t = 0.0;
+    ulonglong2 ad = make_ulonglong2(0ull, 0ull);
     if (g.do_w) {
-      const double t = pixel_nm1(g, ix, iy);
-      tprime[i] = t - g.tc;
+      t = pixel_nm1(g, ix, iy);
       if (screen) {
         // plane k sits at w_k = c0 + k dw: phase_k = c0 t' + k (dw t') turns
         const double c0 = g.w_lo - 0.5 * g.W * g.dw;
-        screen[i] = make_ulonglong2(fixed_turns(c0 * (t - g.tc)), fixed_turns(g.dw * (t - g.tc)));
+        ad = make_ulonglong2(fixed_turns(c0 * (t - g.tc)), fixed_turns(g.dw * (t - g.tc)));
       }
-      // phihat_w(dw t') by quadrature, in the form's own precision
       const R nu = (R)(g.dw * (t - g.tc));
       R ph = (R)0;
       for (int q = 0; q < quad.n; ++q) {
         R s, c;
-        sincos_2pi((R)quad.x[q] * nu, &s, &c);
-        ph += (R)quad.w[q] * c;
+        sincos_2pi(quad.x[q] * nu, &s, &c);
+        ph += quad.w[q] * c;
       }
       f = f / (2.0 * (double)ph * (1.0 + t));
     }
-    corr[i] = (R)f;
+    const int mx = ix > 0 ? g.nx - ix : 0, my = iy > 0 ? g.ny - iy : 0;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      if ((m & 1 && mx == ix) || (m & 2 && my == iy)) continue;  // its own mirror
+      const int64_t o = (int64_t)(m & 2 ? my : iy) * g.nx + (m & 1 ? mx : ix);
+      corr[o] = (R)f;
+      if (tprime) tprime[o] = t - g.tc;
+      if (screen) screen[o] = ad;
+    }
   }
 }
 
@@ -765,20 +782,20 @@ static void make_quadrature(const Geom &g, Quad &q) {
 }
 
 // cu[ix] = 1/phihat((ix - nx/2)/ngx) and cv[iy] likewise, FP64 on the device
-// (keeps the plan's bind free of host copies, so it can be graph-captured).
+// (keeps the plan's bind free of host copies, so it can be graph-captured).  A
+// warp per value, its lanes over the quadrature nodes: one thread's chain of
+// FP64 cosines took 80 us however small the image.
 __global__ void k_corr_1d(const Geom g, const Quad quad, double *__restrict__ cu,
                           double *__restrict__ cv) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.nx + g.ny;
-       i += gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) / 32; i < g.nx + g.ny;
+       i += gridDim.x * blockDim.x / 32) {
     const double nu = i < g.nx ? (double)(i - g.nx / 2) / g.ngx
                                : (double)(i - g.nx - g.ny / 2) / g.ngy;
     double s = 0.0;
-    for (int q = 0; q < quad.n; ++q) s += quad.w[q] * cos(2.0 * M_PI * quad.x[q] * nu);
-    const double f = 1.0 / (2.0 * s);
-    if (i < g.nx)
-      cu[i] = f;
-    else
-      cv[i - g.nx] = f;
+    for (int q = lane; q < quad.n; q += 32) s += quad.w[q] * cospi(2.0 * quad.x[q] * nu);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) (i < g.nx ? cu[i] : cv[i - g.nx]) = 1.0 / (2.0 * s);
   }
 }
 
@@ -867,7 +884,7 @@ static int layout_workspace(gb_plan *p) {
   p->off_corr = off;
   off = align_up(off + rb * (size_t)g.nx * g.ny);
   p->off_tprime = off;
-  off = align_up(off + (g.do_w ? 8 * (size_t)g.nx * g.ny : 0));
+  off = align_up(off + (g.do_w && !p->col_fft ? 8 * (size_t)g.nx * g.ny : 0));
   p->off_screen = off;
   off = align_up(off + (p->col_fft && g.do_w ? 16 * (size_t)g.nx * g.ny : 0));
   p->off_twn = off;
@@ -991,16 +1008,26 @@ static int run_bind(gb_plan *p, cudaStream_t s) {
   // correction factors
   double *tables = p->at<double>(p->off_tables);
   double *cu = tables, *cv = tables + g.nx;
-  k_corr_1d<<<(g.nx + g.ny + kThreads - 1) / kThreads, kThreads, 0, s>>>(g, p->quad, cu, cv);
+  k_corr_1d<<<(g.nx + g.ny + kWarps - 1) / kWarps, kThreads, 0, s>>>(g, p->quad, cu, cv);
   GB_LAUNCH_CHECK("k_corr_1d");
   const int64_t npix = (int64_t)g.nx * g.ny;
-  const unsigned pix_blocks = (unsigned)std::min<int64_t>((npix + kThreads - 1) / kThreads,
+  const int64_t quarter = (int64_t)(g.nx / 2 + 1) * (g.ny / 2 + 1);
+  const unsigned pix_blocks = (unsigned)std::min<int64_t>((quarter + kThreads - 1) / kThreads,
                                                           (int64_t)p->num_sms * 32);
   {
-    ProfScope ps(kProfCorr, s, (double)npix * (sizeof(R) + (g.do_w ? 8.0 : 0.0)));
+    ProfScope ps(kProfCorr, s,
+                 (double)npix * (sizeof(R) + (g.do_w ? (p->col_fft ? 16.0 : 8.0) : 0.0)));
+    QuadIn<R> quad;
+    quad.n = p->quad.n;
+    for (int q = 0; q < quad.n; ++q) {
+      quad.x[q] = (R)p->quad.x[q];
+      quad.w[q] = (R)p->quad.w[q];
+    }
+    // column mode holds the screen's phases, the 2-D transforms' passes n - 1 - tc
     ulonglong2 *screen = p->col_fft && g.do_w ? p->at<ulonglong2>(p->off_screen) : nullptr;
-    k_corr_image<R><<<pix_blocks, kThreads, 0, s>>>(g, cu, cv, p->quad, p->at<R>(p->off_corr),
-                                                     p->at<double>(p->off_tprime), screen);
+    double *tprime = !p->col_fft && g.do_w ? p->at<double>(p->off_tprime) : nullptr;
+    k_corr_image<R><<<pix_blocks, kThreads, 0, s>>>(g, cu, cv, quad, p->at<R>(p->off_corr),
+                                                     tprime, screen);
     GB_LAUNCH_CHECK("k_corr_image");
   }
   if (p->col_fft) {
