@@ -59,7 +59,11 @@ typedef enum { GB_FP32 = 0, GB_FP64 = 1 } gb_precision;
  * pruned to the image's columns and fused with the w-screen, with its own
  * row kernels for power-of-two grid widths from 512 to 16384 (else batched
  * 1-D cuFFT rows); asking for it where it does not apply is GB_ERR_INVALID_ARG.
- * GB_FFT_CUFFT_2D: batched 2-D cuFFT plans plus separate screen passes. */
+ * GB_FFT_CUFFT_2D: 2-D transforms plus separate screen passes; asked for, they
+ * are batched cuFFT plans; where GB_FFT_AUTO comes to them in the FP64 form and
+ * both grid sides are powers of two from 128 to 4096 (the planner raises them
+ * to one, at an oversampling of its choice, where that is faster), the
+ * library's own transforms, which skip what holds no data. */
 typedef enum { GB_FFT_AUTO = 0, GB_FFT_CUFFT_2D = 1, GB_FFT_COLUMNS = 2 } gb_fft_mode;
 
 /* Image memory layout.  GB_LAYOUT_XY is ducc0's dirty[x][y] (what

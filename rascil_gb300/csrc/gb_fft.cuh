@@ -44,6 +44,14 @@ int setup_row_kernels(gb_plan *p);
 // (e^{+}, occupied bins in, image columns out), dir < 0 predict (e^{-}, image
 // columns in, occupied bins out); rows without occupied bins are skipped.
 int run_rows(gb_plan *p, void *grid, int b0, int nb, int dir, cudaStream_t s);
+// FP64 form, power-of-two grids (gb_fft64.cu): line lengths with a k_fft64
+// instantiation for an image of n cells (the middle half at most); opt-ins and
+// twiddle tables; the pruned 2-D transform of nb planes x NP pols, dir as above
+// (invert leaves the image block, predict reads it).
+bool fft64_fits(int ng, int n);
+int setup_fft64(gb_plan *p);
+int init_fft64(gb_plan *p, cudaStream_t s);
+int run_fft64(gb_plan *p, int b0, int nb, void *grid, int dir, cudaStream_t s);
 // Invert: step A in place, then step B fused with the w-screen and the
 // image accumulation (first != 0 starts acc from zero).
 int run_cols_invert(gb_plan *p, void *grid, int b0, int nb, float *acc, int first,

@@ -507,15 +507,14 @@ __global__ void __launch_bounds__(kThreads)
     for (int p = 0; p < NP; ++p) a[p] = first ? (R)0 : acc[p * npix + i];
     const size_t gi = (size_t)(iy + oy) * g.ngx + (ix + ox);
     if (g.do_w) {
-      PlaneTurns pt;
-      pt.start(g, b0, tprime[i]);
+      PlaneScreen<R> ps;
+      ps.start(g, b0, tprime[i]);
       for (int j = 0; j < nb; ++j) {
-        R s, c;
-        sincos_2pi(pt.turns(j, (R)0), &s, &c);
+        ps.plane(j);
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
           const C v = grid[((size_t)j * NP + p) * plane + gi];
-          a[p] += v.x * c + v.y * s;
+          a[p] += v.x * ps.c + v.y * ps.s;
         }
       }
     } else {
@@ -634,9 +633,9 @@ static int inv_zero_impl(gb_plan *p, int bi, cudaStream_t s) {
   C *grid = reinterpret_cast<C *>(p->ws + p->off_temp + p->c_grid);
   const int b0 = bi * g.B, nb = std::min(g.B, g.nplanes - b0);
   const double gbytes = (double)sizeof(C) * nb * NP * (double)g.ngx * g.ngy;
-  if (p->col_fft) {  // only what the gridder writes; the transforms skip the rest
+  if (p->col_fft || p->fft64) {  // only what the gridder writes; the transforms skip the rest
     ProfScope ps(kProfGridZero, s,
-                 (p->row_fft ? p->used_cells(b0, nb) : p->used_rows(b0, nb)) * gbytes);
+                 (p->row_fft || p->fft64 ? p->used_cells(b0, nb) : p->used_rows(b0, nb)) * gbytes);
     return run_zero_rows(p, grid, b0, nb, s);
   }
   ProfScope ps(kProfGridZero, s, gbytes);
@@ -707,6 +706,12 @@ static int inv_transform_impl(gb_plan *p, int bi, cudaStream_t s) {
     ProfScope ps(kProfRowsInv, s,
                  (p->used_cells(b0, nb) + 0.5 * p->used_rows(b0, nb)) * gbytes);
     rc = run_rows(p, grid, b0, nb, 1, s);
+  } else if (p->fft64) {
+    // occupied bins, then the image columns of the used rows, read; those
+    // columns, then the image, written
+    ProfScope ps(kProfFftInv, s,
+                 (p->used_cells(b0, nb) + p->used_rows(b0, nb) + 0.25) * gbytes);
+    rc = run_fft64(p, b0, nb, grid, 1, s);
   } else {
     ProfScope ps(kProfFftInv, s, 2.0 * gbytes);
     rc = run_fft(p, nb, grid, CUFFT_INVERSE, s);

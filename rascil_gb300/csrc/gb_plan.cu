@@ -58,7 +58,7 @@ static int good_size(int n) {
 }
 
 static int plan_geometry_sigma(const gb_plan_params *p, double w_lo, double w_hi, double sigma,
-                               Geom &g);
+                               Geom &g, bool pad = false);
 
 // Cost model of one direction (invert or predict) of a plan, in seconds on
 // GB300, for choosing the grid oversampling when the caller leaves it at 0
@@ -81,6 +81,23 @@ static bool columns_apply(const gb_plan_params *p, const Geom &g) {
   int n1, n2;
   return p->precision == GB_FP32 && p->fft_mode != GB_FFT_CUFFT_2D && g.ngy == 2 * g.ny &&
          (g.ngx - g.nx) % 4 == 0 && column_split(g.ngy, n1, n2);
+}
+
+// The FP64 form's own transforms (gb_fft64.cu).
+static bool fft64_applies(const gb_plan_params *p, const Geom &g) {
+  return p->precision == GB_FP64 && fft64_fits(g.ngx, g.nx) && fft64_fits(g.ngy, g.ny);
+}
+
+// Per cell of a w-plane, FP64 form: cuFFT's full transform of a grid that is no
+// power of two (measured 2.2e-10 s at 972^2, whose factors are 4 3^5; 1.0e-10 at
+// 1024^2), and the library's pruned one of a power of two (5.4e-11 at 1024^2,
+// 4.3e-11 at 2048^2).
+constexpr double kCostCell64Cufft = 1.8e-10, kCostCell64Own = 6.0e-11;
+
+static int next_pow2(int n) {
+  int m = 1;
+  while (m < n) m *= 2;
+  return m;
 }
 
 static double plan_cost(const gb_plan_params *p, const Geom &g) {
@@ -117,12 +134,22 @@ int plan_geometry(const gb_plan_params *p, double w_lo, double w_hi, Geom &g) {
     }
   }
   if (!found) return plan_geometry_sigma(p, w_lo, w_hi, 2.0, g);  // for its error message
+  // the FP64 form at that oversampling: sides raised to powers of two where the
+  // library's own transforms of the larger grid cost less than cuFFT's of the
+  // smaller (the wider oversampling only lowers the aliasing error)
+  if (p->precision == GB_FP64 && p->fft_mode == GB_FFT_AUTO && !fft64_applies(p, g)) {
+    Geom t;
+    if (plan_geometry_sigma(p, w_lo, w_hi, g.sigma, t, true) == GB_OK && fft64_applies(p, t) &&
+        kCostCell64Own * t.ngx * t.ngy < kCostCell64Cufft * g.ngx * g.ngy)
+      g = t;
+  }
   set_error("");
   return GB_OK;
 }
 
+// `pad`: grid sides raised to powers of two.
 static int plan_geometry_sigma(const gb_plan_params *p, double w_lo, double w_hi, double sigma,
-                               Geom &g) {
+                               Geom &g, bool pad) {
   if (p->nrows <= 0 || p->nchan <= 0) {
     set_error("nrows and nchan must be positive (got %lld, %d)", (long long)p->nrows,
               p->nchan);
@@ -212,6 +239,10 @@ static int plan_geometry_sigma(const gb_plan_params *p, double w_lo, double w_hi
   g.do_w = p->do_wstacking ? 1 : 0;
   g.ngx = good_size(std::max((int)std::ceil(sigma * p->npix_x), 2 * W));
   g.ngy = good_size(std::max((int)std::ceil(sigma * p->npix_y), 2 * W));
+  if (pad) {
+    g.ngx = next_pow2(g.ngx);
+    g.ngy = next_pow2(g.ngy);
+  }
   const double xm = 0.5 * p->npix_x * p->pixsize_x;
   const double ym = 0.5 * p->npix_y * p->pixsize_y;
   const double r2 = xm * xm + ym * ym;
@@ -600,7 +631,8 @@ __global__ void k_corr_image(const Geom g, const double *__restrict__ cu,
 // order of first w-plane) reach planes from its first item's first to its
 // last item's last, rows [tv T, tv T + T + W - 1) and columns [tu T, tu T + T + W - 1)
 // (mod the grid).
-__global__ void k_row_mask(const Geom g, const ItemF *__restrict__ items,
+template <typename Item>
+__global__ void k_row_mask(const Geom g, const Item *__restrict__ items,
                            const Chunk *__restrict__ chunks,
                            const uint32_t *__restrict__ chunk_off, uint32_t *__restrict__ mask) {
   const uint32_t nch = chunk_off[g.nbuckets];
@@ -863,6 +895,7 @@ static int choose_fft_mode(gb_plan *p) {
       return GB_ERR_INVALID_ARG;
   }
   p->row_fft = p->col_fft && row_kernel_fits(p->g.ngx, p->g.nx);
+  p->fft64 = p->params.fft_mode == GB_FFT_AUTO && fft64_applies(&p->params, p->g);
   return GB_OK;
 }
 
@@ -888,11 +921,11 @@ static int layout_workspace(gb_plan *p) {
   p->off_screen = off;
   off = align_up(off + (p->col_fft && g.do_w ? 16 * (size_t)g.nx * g.ny : 0));
   p->off_twn = off;
-  off = align_up(off + (p->col_fft ? 8 * (size_t)g.ngy : 0));
+  off = align_up(off + (p->col_fft ? 8 : p->fft64 ? 16 : 0) * (size_t)g.ngy);
   p->off_twx = off;
-  off = align_up(off + (p->row_fft ? 8 * (size_t)g.ngx : 0));
+  off = align_up(off + (p->row_fft ? 8 : p->fft64 ? 16 : 0) * (size_t)g.ngx);
   p->off_rowmask = off;
-  off = align_up(off + (p->col_fft ? 4 * (size_t)g.nplanes * g.ntv : 0));
+  off = align_up(off + (p->col_fft || p->fft64 ? 4 * (size_t)g.nplanes * g.ntv : 0));
   p->off_tables = off;
   off = align_up(off + 8 * ((size_t)g.nx + g.ny + 2 * kMaxQuad));
   // shifted plans keep uvw and f/c: a PSF call rebuilds the unshifted factor
@@ -1040,12 +1073,16 @@ static int run_bind(gb_plan *p, cudaStream_t s) {
                                                                      p->at<float2>(p->off_twx));
     GB_LAUNCH_CHECK("k_twiddles");
   }
-  if (p->col_fft) {
+  if (p->fft64) {
+    rc = init_fft64(p, s);
+    if (rc) return rc;
+  }
+  if (p->col_fft || p->fft64) {
     uint32_t *mask = p->at<uint32_t>(p->off_rowmask);
     GB_CUDA(cudaMemsetAsync(mask, 0, 4 * (size_t)g.nplanes * g.ntv, s));
     const unsigned cb = (unsigned)std::min<int64_t>(
         ((int64_t)p->max_chunks + kThreads - 1) / kThreads, (int64_t)p->num_sms * 16);
-    k_row_mask<<<cb, kThreads, 0, s>>>(g, p->at<ItemF>(p->off_items), chunks, chunk_off, mask);
+    k_row_mask<Item><<<cb, kThreads, 0, s>>>(g, items, chunks, chunk_off, mask);
     GB_LAUNCH_CHECK("k_row_mask");
     if (prof_on()) {  // host copy for the profiler's byte counts (costs a sync)
       p->mask_host.assign((size_t)g.nplanes * g.ntv, 0);
@@ -1222,7 +1259,8 @@ int gb_plan_create(const gb_plan_params *params, const double *uvw_dev,
     return rc;
   }
   p->rem_planes = p->g.nplanes % p->g.B;
-  if (!p->row_fft) {
+  const bool own = p->row_fft || p->fft64;
+  if (!own) {
     rc = make_fft(p, p->g.B, &p->fft_full, &w_full);
     if (rc) {
       gb_plan_destroy(p);
@@ -1230,7 +1268,7 @@ int gb_plan_create(const gb_plan_params *params, const double *uvw_dev,
     }
     p->fft_full_ok = true;
   }
-  if (p->rem_planes && !p->row_fft) {
+  if (p->rem_planes && !own) {
     rc = make_fft(p, p->rem_planes, &p->fft_rem, &w_rem);
     if (rc) {
       gb_plan_destroy(p);
@@ -1246,6 +1284,7 @@ int gb_plan_create(const gb_plan_params *params, const double *uvw_dev,
   rc = setup_tile_kernels(p);
   if (!rc) rc = setup_col_kernels(p);
   if (!rc) rc = setup_row_kernels(p);
+  if (!rc) rc = setup_fft64(p);
   if (rc) {
     gb_plan_destroy(p);
     return rc;

@@ -42,6 +42,9 @@ struct gb_plan {
   // column mode with rows of 512 to 16384 cells (powers of two): the row
   // transforms are k_rows (no cuFFT plan), which follow the occupancy mask
   bool row_fft = false;
+  // FP64 form, power-of-two grids: the transforms are k_fft64 (no cuFFT plan),
+  // which follow the occupancy mask as well
+  bool fft64 = false;
   size_t off_rowmask = 0, off_twx = 0;
   int row_blocks = 0;
   size_t off_tprime = 0;  // [ny][nx] float64: n - 1 - tc per pixel (w-stacking, 2-D transforms)

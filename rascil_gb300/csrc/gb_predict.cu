@@ -54,6 +54,42 @@ __global__ void k_prep_image(const Geom g, const R *__restrict__ dirty, int layo
   }
 }
 
+// The screened image into the image block of every plane (k_fft64 reads nothing
+// else of it).
+template <typename R, int NP>
+__global__ void __launch_bounds__(kThreads)
+    k_screen_block(const Geom g, const R *__restrict__ img, const double *__restrict__ tprime,
+                   int b0, int nb, typename Traits<R>::C *__restrict__ grid) {
+  using C = typename Traits<R>::C;
+  const int64_t npix = (int64_t)g.nx * g.ny, plane = (int64_t)g.ngx * g.ngy;
+  const int ox = (g.ngx - g.nx) / 2, oy = (g.ngy - g.ny) / 2;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < npix; i += stride) {
+    const int iy = (int)(i / g.nx), ix = (int)(i - (int64_t)iy * g.nx);
+    C *dst = grid + (int64_t)(iy + oy) * g.ngx + ix + ox;
+    R v[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) v[p] = img[p * npix + i];
+    PlaneScreen<R> ps;
+    if (g.do_w) ps.start(g, b0, tprime[i]);
+    for (int j = 0; j < nb; ++j) {
+      if (g.do_w) {
+        ps.plane(j);
+      } else {
+        ps.c = (R)1;
+        ps.s = (R)0;
+      }
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        C z;
+        z.x = v[p] * ps.c;
+        z.y = v[p] * ps.s;
+        dst[((int64_t)j * NP + p) * plane] = z;
+      }
+    }
+  }
+}
+
 template <typename R, int NP>
 __global__ void __launch_bounds__(kThreads)
     k_screen_pad(const Geom g, const R *__restrict__ img, const double *__restrict__ tprime,
@@ -72,16 +108,15 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
       for (int p = 0; p < NP; ++p) v[p] = img[p * npix + pi];
       if (g.do_w) {
-        PlaneTurns pt;
-        pt.start(g, b0, tprime[pi]);
+        PlaneScreen<R> ps;
+        ps.start(g, b0, tprime[pi]);
         for (int j = 0; j < nb; ++j) {
-          R s, c;
-          sincos_2pi(pt.turns(j, (R)0), &s, &c);
+          ps.plane(j);
 #pragma unroll
           for (int p = 0; p < NP; ++p) {
             C z;
-            z.x = v[p] * c;
-            z.y = v[p] * s;
+            z.x = v[p] * ps.c;
+            z.y = v[p] * ps.s;
             grid[((int64_t)j * NP + p) * plane + i] = z;
           }
         }
@@ -505,6 +540,23 @@ static int pred_transform_impl(gb_plan *p, int bi, cudaStream_t s) {
       const int rc = run_cols_predict(p, img, b0, nb, grid, s);
       if (rc) return rc;
       cols = true;
+    }
+  }
+  if (p->fft64) {
+    if constexpr (std::is_same<R, double>::value) {
+      {
+        const unsigned pix_blocks = (unsigned)std::min<int64_t>(
+            ((int64_t)npix + kThreads - 1) / kThreads, (int64_t)p->num_sms * 32);
+        ProfScope ps(kProfScreenPad, s, 0.25 * gbytes + sizeof(R) * NP * npix);
+        k_screen_block<R, NP><<<pix_blocks, kThreads, 0, s>>>(
+            g, img, p->at<double>(p->off_tprime), b0, nb, grid);
+        GB_LAUNCH_CHECK("k_screen_block");
+      }
+      // the image, then the image columns of the used rows, read; those
+      // columns, then the occupied bins, written
+      ProfScope ps(kProfFftFwd, s,
+                   (p->used_cells(b0, nb) + p->used_rows(b0, nb) + 0.25) * gbytes);
+      return run_fft64(p, b0, nb, grid, -1, s);
     }
   }
   if (!cols) {

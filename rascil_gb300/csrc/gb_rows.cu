@@ -453,10 +453,10 @@ __global__ void __launch_bounds__(RowLayout<N>::TH, RowShape<N>::MINB) k_rows(co
   }
 }
 
-// Zero the occupied bins (whole rows of occupied tiles when `bw` is 0) of
-// nrows = nb NP ngy rows of ngx cells: a warp per row.
-__global__ void k_zero_rows(float2 *__restrict__ grid, const uint32_t *__restrict__ mask,
-                            int64_t nrows, int ngx, int ngy, int NP, int b0, int T, int ntv,
+// Zero the occupied bins of `bw` 16-byte units (whole rows of occupied tiles when
+// bw is 0) of nrows = nb NP ngy rows of `width` units: a warp per row.
+__global__ void k_zero_rows(float4 *__restrict__ grid, const uint32_t *__restrict__ mask,
+                            int64_t nrows, int width, int ngy, int NP, int b0, int T, int ntv,
                             int bw) {
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * (blockDim.x / 32);
@@ -464,16 +464,16 @@ __global__ void k_zero_rows(float2 *__restrict__ grid, const uint32_t *__restric
        row += stride) {
     const int sp = (int)(row / ngy), r = (int)(row - (int64_t)sp * ngy);
     uint32_t occ = mask[(int64_t)(b0 + sp / NP) * ntv + r / T];
-    float4 *dst = reinterpret_cast<float4 *>(grid + row * ngx);
+    float4 *dst = grid + row * width;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     if (bw == 0) {
       if (occ)
-        for (int i = lane; i < ngx / 2; i += 32) dst[i] = zero;
+        for (int i = lane; i < width; i += 32) dst[i] = zero;
       continue;
     }
     for (; occ; occ &= occ - 1) {
-      float4 *p = dst + (__ffs(occ) - 1) * (bw / 2);
-      for (int i = lane; i < bw / 2; i += 32) p[i] = zero;
+      float4 *p = dst + (__ffs(occ) - 1) * bw;
+      for (int i = lane; i < bw; i += 32) p[i] = zero;
     }
   }
 }
@@ -484,9 +484,10 @@ int run_zero_rows(gb_plan *p, void *grid, int b0, int nb, cudaStream_t s) {
   const unsigned blocks =
       (unsigned)std::min<int64_t>((nrows + kWarps - 1) / kWarps, (int64_t)p->num_sms * 8);
   // the row kernels read the occupied bins only; cuFFT rows read whole rows
-  k_zero_rows<<<blocks, kThreads, 0, s>>>(reinterpret_cast<float2 *>(grid),
-                                          p->at<uint32_t>(p->off_rowmask), nrows, g.ngx, g.ngy,
-                                          g.NP, b0, g.T, g.ntv, p->row_fft ? g.ngx / 32 : 0);
+  const int width = p->fft64 ? g.ngx : g.ngx / 2;
+  k_zero_rows<<<blocks, kThreads, 0, s>>>(
+      reinterpret_cast<float4 *>(grid), p->at<uint32_t>(p->off_rowmask), nrows, width, g.ngy,
+      g.NP, b0, g.T, g.ntv, p->row_fft || p->fft64 ? width / 32 : 0);
   GB_LAUNCH_CHECK("k_zero_rows");
   return GB_OK;
 }
