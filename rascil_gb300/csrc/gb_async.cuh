@@ -1,5 +1,5 @@
-// Asynchronous copies for the tile kernels: cp.async (8-byte, per thread)
-// and TMA bulk tensor copies completing on shared-memory mbarriers.
+// Asynchronous copies: cp.async (16-byte, per thread), and TMA bulk and bulk tensor
+// copies completing on shared-memory mbarriers.
 #pragma once
 
 #include <cuda.h>
@@ -7,17 +7,17 @@
 
 namespace gb {
 
-__device__ __forceinline__ void cp_async8(void *smem_dst, const void *gmem_src, bool valid) {
+__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src) {
   const unsigned dst = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(gmem_src),
-               "r"(valid ? 8 : 0)
-               : "memory");
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(gmem_src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+// Until at most N of this thread's groups are in flight.
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 
-// TMA (bulk tensor copies) with mbarrier completion.
+// TMA (bulk copies) with mbarrier completion.
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
   return (unsigned)__cvta_generic_to_shared(p);
 }

@@ -644,7 +644,8 @@ __global__ void k_row_mask(const Geom g, const Item *__restrict__ items,
     const int tile = (int)(ch.bucket - (uint32_t)slab * ntiles);
     const int tv = tile / g.ntu, tu = tile - tv * g.ntu;
     uint32_t bits = 0;
-    const int c_hi = tu * g.T + g.T + g.W - 2;  // inclusive
+    // inclusive; rounded up to a whole pair of cells (the degridder stages pairs)
+    const int c_hi = (tu * g.T + g.T + g.W - 2) | 1;
     for (int x = tu * g.T; x <= c_hi + bw - 1; x += bw) {
       int xx = min(x, c_hi);
       while (xx >= g.ngx) xx -= g.ngx;
