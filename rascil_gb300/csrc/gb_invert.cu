@@ -392,6 +392,7 @@ __device__ __forceinline__ void grid_chunk(
     // threads in order; a thread's next pair is step_row rows and step_pair pairs on
     const int hp = (SW + 1) >> 1, step_row = kThreads / hp, step_pair = kThreads - step_row * hp;
     const int row_0 = threadIdx.x / hp, pair_0 = threadIdx.x - row_0 * hp;
+    const bool even = (T & 1) == 0;
     __syncthreads();
     for (int k = k_lo; k < k_hi; ++k) {
       float2 *gplane = grid + (size_t)(k - b0) * NP * plane;
@@ -437,11 +438,11 @@ __device__ __forceinline__ void grid_chunk(
       if (!direct) {
         __syncthreads();
         // flush: fixed point -> float, add to HBM, and leave the sub-grid
-        // zeroed.  A thread takes two adjacent cells (x even): one 16-byte
-        // vector atomic per pol for both (tile origins, x and the grid width
-        // are even, so p is even and the pair never straddles the wrap).  For
-        // odd SW the last pair's second cell is row padding, never written,
-        // so it adds zero.
+        // zeroed.  A thread takes two adjacent cells (x even): with an even
+        // tile side one 16-byte vector atomic per pol for both (tile origins, x
+        // and the grid width are even, so p is even and the pair never straddles
+        // the wrap), with an odd one an 8-byte atomic each.  For odd SW the last
+        // pair's second cell is row padding, never written, so it adds zero.
         for (int y = row_0, pair = pair_0; y < SW;) {
           const int cell = y * L.pitch + 2 * pair;
           int p = tu * T + 2 * pair;
@@ -459,8 +460,14 @@ __device__ __forceinline__ void grid_chunk(
             if ((re.x | re.y | im.x | im.y) != 0) {
               *are = make_int2(0, 0);
               *aim = make_int2(0, 0);
-              grid_add2(dst + pol * plane, inv * (float)re.x, inv * (float)im.x,
-                        inv * (float)re.y, inv * (float)im.y);
+              const float re0 = inv * (float)re.x, im0 = inv * (float)im.x;
+              const float re1 = inv * (float)re.y, im1 = inv * (float)im.y;
+              if (even) {
+                grid_add2(dst + pol * plane, re0, im0, re1, im1);
+              } else {  // the second cell may be the next row's first (the wrap)
+                grid_add(dst + pol * plane, re0, im0);
+                grid_add((p + 1 < g.ngx ? dst + 1 : dst + 1 - g.ngx) + pol * plane, re1, im1);
+              }
             }
           }
           pair += step_pair;
