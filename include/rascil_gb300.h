@@ -62,8 +62,9 @@ typedef enum { GB_FP32 = 0, GB_FP64 = 1 } gb_precision;
  * GB_FFT_CUFFT_2D: 2-D transforms plus separate screen passes; asked for, they
  * are batched cuFFT plans; where GB_FFT_AUTO comes to them in the FP64 form and
  * both grid sides are powers of two from 128 to 4096 (the planner raises them
- * to one, at an oversampling of its choice, where that is faster), the
- * library's own transforms, which skip what holds no data. */
+ * to one, at an oversampling of its choice and an epsilon of 1e-9 or below,
+ * where that is faster), the library's own transforms, which skip what holds
+ * no data. */
 typedef enum { GB_FFT_AUTO = 0, GB_FFT_CUFFT_2D = 1, GB_FFT_COLUMNS = 2 } gb_fft_mode;
 
 /* Image memory layout.  GB_LAYOUT_XY is ducc0's dirty[x][y] (what

@@ -94,6 +94,8 @@ static bool fft64_applies(const gb_plan_params *p, const Geom &g) {
 // 4.3e-11 at 2048^2).
 constexpr double kCostCell64Cufft = 1.8e-10, kCostCell64Own = 6.0e-11;
 
+constexpr double kPadEpsilon = 1e-9;
+
 static int next_pow2(int n) {
   int m = 1;
   while (m < n) m *= 2;
@@ -136,8 +138,11 @@ int plan_geometry(const gb_plan_params *p, double w_lo, double w_hi, Geom &g) {
   if (!found) return plan_geometry_sigma(p, w_lo, w_hi, 2.0, g);  // for its error message
   // the FP64 form at that oversampling: sides raised to powers of two where the
   // library's own transforms of the larger grid cost less than cuFFT's of the
-  // smaller (the wider oversampling only lowers the aliasing error)
-  if (p->precision == GB_FP64 && p->fft_mode == GB_FFT_AUTO && !fft64_applies(p, g)) {
+  // smaller (the wider oversampling only lowers the aliasing error).  Another grid
+  // moves the result by up to epsilon: only where that is at the level FP64
+  // results are compared at
+  if (p->precision == GB_FP64 && p->epsilon <= kPadEpsilon && p->fft_mode == GB_FFT_AUTO &&
+      !fft64_applies(p, g)) {
     Geom t;
     if (plan_geometry_sigma(p, w_lo, w_hi, g.sigma, t, true) == GB_OK && fft64_applies(p, t) &&
         kCostCell64Own * t.ngx * t.ngy < kCostCell64Cufft * g.ngx * g.ngy)
