@@ -94,22 +94,77 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// exp(2 pi i d s) in FP64 (d metres, s wavelengths per metre) from a table of
+// kTurnTable points on the circle and a short series.  In units of a table step,
+// d S = m + r with S = kTurnTable s, m an integer and |r| <= 1/2: r is one fused
+// multiply-add, so the product d S is never rounded, and S's own rounding goes
+// back in by its low part; exp of r steps by its Taylor polynomial (the first
+// terms left out are below 1e-17), times the table's entry m.  15 FP64 instructions
+// (16 cycles of the SM's FP64 pipe each) where sincospi with its argument
+// reduction takes about 30.  m comes out of the low bits of d S + 1.5 2^52
+// (|d S| < 2^50).
+constexpr int kTurnTable = 256;
+
+__device__ __forceinline__ void turn_table(double2 *tab) {
+  for (int i = threadIdx.x; i < kTurnTable; i += blockDim.x) {
+    double s, c;
+    sincospi(2.0 * i / kTurnTable, &s, &c);
+    tab[i] = make_double2(c, s);
+  }
+}
+
+// S = kTurnTable f / c as a double and what that leaves out; f = f_hi + f_lo.
+struct TurnScale {
+  double hi, lo;
+  __device__ __forceinline__ TurnScale(double f_hi, double f_lo) {
+    const double s = f_hi / kSpeedOfLight;
+    hi = s * kTurnTable;  // exact: a power of two
+    lo = (fma(-s, kSpeedOfLight, f_hi) + f_lo) / kSpeedOfLight * kTurnTable;
+  }
+};
+
+__device__ __forceinline__ double2 exp_turns(double d, const TurnScale &s, const double2 *tab) {
+  constexpr double kMagic = 6755399441055744.0;              // 1.5 2^52
+  constexpr double kStep = 6.2831853071795864769 / kTurnTable;  // radians per step
+  constexpr double k2 = kStep * kStep, k4 = k2 * k2;
+  const double m = fma(d, s.hi, kMagic);
+  const double r = fma(d, s.lo, fma(d, s.hi, -(m - kMagic))), r2 = r * r;
+  const double sn = fma(fma(kStep * k4 / 120.0, r2, -kStep * k2 / 6.0), r2, kStep) * r;
+  const double cs = fma(fma(fma(-k4 * k2 / 720.0, r2, k4 / 24.0), r2, -k2 / 2.0), r2, 1.0);
+  const double2 w = tab[__double2loint(m) & (kTurnTable - 1)];
+  return make_double2(fma(w.x, cs, -(w.y * sn)), fma(w.x, sn, w.y * cs));
+}
+
 // Uniformly spaced channels (f_c = f_0 + c df): for a row and a component the
-// phase is linear in c, so exp(-2 pi i turns(c)) = base * step^c.  One thread
-// per (row, block of CB channels) evaluates two FP64 sincospi per component
-// and then one complex multiply per channel instead of a sincos; the
-// recurrence adds about one rounding per channel (< 1e-14 relative over CB).
+// phase is linear in c.  One thread per (row, block of CB channels) evaluates
+// exp(-2 pi i turns) at the block's middle channel and the channel step, and goes
+// outwards both ways by x_(j+1) = 2 cos(step) x_j - x_(j-1) (two FP64 instructions a
+// channel instead of a complex product's four; about j (j + 1) / 2 roundings after j <=
+// CB / 2 steps, no more than CB successive products have).  The kernel is bound
+// by FP64 instructions: 3 for the row and component, 30 for the two exponentials,
+// 18 for the eight channels and 4 per channel and pol for the sum.  65,024 rows x 8
+// channels x 200 components x 1 pol: 3.9 ms with two sincospi and successive
+// products in blocks of 256 threads (two waves of blocks on 152 SMs), 2.4 ms so, in
+// blocks of 64.
+constexpr int kDftThreads = 64;
+
 template <typename OutC, int P, int CB>
-__global__ void __launch_bounds__(kThreads)
-    k_dft_components_uniform(const double *__restrict__ uvw, double f0, double df,
-                             int64_t nrows, int nchan, const double *__restrict__ lmn,
+__global__ void __launch_bounds__(kDftThreads)
+    k_dft_components_uniform(const double *__restrict__ uvw, const double *__restrict__ freq,
+                             double df, int64_t nrows, int nchan, const double *__restrict__ lmn,
                              const double2 *__restrict__ flux, int ncomp,
                              OutC *__restrict__ vis) {
+  constexpr int H = CB / 2;  // channel c0 + H is the middle one
   __shared__ double s_lmn[kDftTile][3];
+  __shared__ double2 s_tab[kTurnTable];
+  turn_table(s_tab);
   const int c0 = blockIdx.y * CB;
   const int nc = min(CB, nchan - c0);
-  const double s0 = (f0 + c0 * df) / kSpeedOfLight;
-  const double ds = df / kSpeedOfLight;
+  // the middle channel's frequency as given (a block cut short by the last
+  // channel: that many steps past it, the sum's rounding kept)
+  const int cm = min(c0 + H, nchan - 1);
+  const double past = (c0 + H - cm) * df, fm = freq[cm] + past;
+  const TurnScale s0(fm, past - (fm - freq[cm])), ds(df, 0.0);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < nrows; base += stride) {
     const int64_t r = base + threadIdx.x;
@@ -128,15 +183,30 @@ __global__ void __launch_bounds__(kThreads)
       __syncthreads();
       if (!active) continue;
       for (int k = 0; k < nk; ++k) {
-        const double d = u * s_lmn[k][0] + v * s_lmn[k][1] + w * s_lmn[k][2];
-        double t0 = d * s0, dt = d * ds;
-        t0 -= rint(t0);
-        dt -= rint(dt);
-        double bs, bc, ss, sc;
-        sincospi(2.0 * t0, &bs, &bc);
-        sincospi(2.0 * dt, &ss, &sc);
-        double pr = bc, pi = -bs;         // exp(-2 pi i t0)
-        const double qr = sc, qi = -ss;   // exp(-2 pi i dt)
+        const double d = -(u * s_lmn[k][0] + v * s_lmn[k][1] + w * s_lmn[k][2]);
+        const double2 a = exp_turns(d, s0, s_tab), q = exp_turns(d, ds, s_tab);
+        double xr[CB], xi[CB];  // exp(-2 pi i turns) per channel
+        xr[H] = a.x;
+        xi[H] = a.y;
+        // the neighbours a q and a conj(q) share their four products
+        const double rr = a.x * q.x, ri = a.x * q.y;
+        if (H + 1 < CB) {
+          xr[H + 1] = fma(-a.y, q.y, rr);
+          xi[H + 1] = fma(a.y, q.x, ri);
+        }
+        xr[H - 1] = fma(a.y, q.y, rr);
+        xi[H - 1] = fma(a.y, q.x, -ri);
+        const double c2 = 2.0 * q.x;
+#pragma unroll
+        for (int c = H + 2; c < CB; ++c) {
+          xr[c] = fma(c2, xr[c - 1], -xr[c - 2]);
+          xi[c] = fma(c2, xi[c - 1], -xi[c - 2]);
+        }
+#pragma unroll
+        for (int c = H - 2; c >= 0; --c) {
+          xr[c] = fma(c2, xr[c + 1], -xr[c + 2]);
+          xi[c] = fma(c2, xi[c + 1], -xi[c + 2]);
+        }
         const double2 *f = flux + ((size_t)(k0 + k) * nchan + c0) * P;
 #pragma unroll
         for (int c = 0; c < CB; ++c) {
@@ -144,13 +214,10 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
             for (int p = 0; p < P; ++p) {
               const double2 fl = f[c * P + p];
-              ar[c][p] += fl.x * pr - fl.y * pi;
-              ai[c][p] += fl.x * pi + fl.y * pr;
+              ar[c][p] += fl.x * xr[c] - fl.y * xi[c];
+              ai[c][p] += fl.x * xi[c] + fl.y * xr[c];
             }
           }
-          const double nr = pr * qr - pi * qi;
-          pi = pr * qi + pi * qr;
-          pr = nr;
         }
       }
     }
@@ -263,12 +330,12 @@ int gb_dft_components(const double *uvw, const double *freq, int64_t nrows, int3
   if (uniform) {
     constexpr int CB4 = 4, CB8 = 8;
     const int cb = npol == 4 ? CB4 : CB8;
-    const unsigned rblocks = (unsigned)std::min<int64_t>((nrows + kThreads - 1) / kThreads,
-                                                         (int64_t)sms * 8);
+    const unsigned rblocks = (unsigned)std::min<int64_t>((nrows + kDftThreads - 1) / kDftThreads,
+                                                         (int64_t)sms * 32);
     dim3 grid(rblocks, (unsigned)((nchan + cb - 1) / cb));
 #define GB_DFTU(OutC, P, CB)                                                                  \
-  k_dft_components_uniform<OutC, P, CB><<<grid, kThreads, 0, s>>>(                             \
-      uvw, f0, df, nrows, nchan, lmn, f, ncomp, reinterpret_cast<OutC *>(vis))
+  k_dft_components_uniform<OutC, P, CB><<<grid, kDftThreads, 0, s>>>(                           \
+      uvw, freq, df, nrows, nchan, lmn, f, ncomp, reinterpret_cast<OutC *>(vis))
     if (vis_precision == GB_FP64) {
       if (npol == 1) GB_DFTU(double2, 1, CB8);
       else if (npol == 2) GB_DFTU(double2, 2, CB8);
