@@ -43,6 +43,37 @@ bool sync_check_enabled() {
   return on;
 }
 
+cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t s) {
+  static std::mutex lock;
+  static std::vector<cudaMemPool_t> pools;  // by device; null where none could be made
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> hold(lock);
+    while ((int)pools.size() <= dev) {
+      cudaMemPoolProps props;
+      memset(&props, 0, sizeof(props));
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = (int)pools.size();
+      cudaMemPool_t made = nullptr;
+      uint64_t keep = (uint64_t)32 << 20;  // a pool grows by 2 MiB and more at a time
+      if (cudaMemPoolCreate(&made, &props) != cudaSuccess ||
+          cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        made = nullptr;
+      }
+      pools.push_back(made);
+    }
+    pool = pools[dev];
+  }
+  if (pool && cudaMallocFromPoolAsync(ptr, bytes, pool, s) == cudaSuccess) return cudaSuccess;
+  if (pool) cudaGetLastError();
+  return cudaMallocAsync(ptr, bytes, s);
+}
+
 // ---------------------------------------------------------------------
 // Host planning
 
@@ -459,6 +490,31 @@ __global__ void k_wrange(const double *__restrict__ uvw, int64_t nrows, int mirr
   }
 }
 
+// The partials' totals and the frequencies side by side in `out` (3 + nchan), so
+// that one copy brings both to the host.
+__global__ void k_wrange_end(const double *__restrict__ part, int nparts,
+                             const double *__restrict__ freq, int nchan,
+                             double *__restrict__ out) {
+  for (int c = threadIdx.x; c < nchan; c += blockDim.x) out[3 + c] = freq[c];
+  if (threadIdx.x >= 32) return;
+  double lo = INFINITY, hi = -INFINITY, bad = 0.0;
+  for (int i = threadIdx.x; i < nparts; i += 32) {
+    lo = fmin(lo, part[3 * i]);
+    hi = fmax(hi, part[3 * i + 1]);
+    bad += part[3 * i + 2];
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    bad += __shfl_xor_sync(0xffffffffu, bad, o);
+  }
+  if (threadIdx.x == 0) {
+    out[0] = lo;
+    out[1] = hi;
+    out[2] = bad;
+  }
+}
+
 // ---------------------------------------------------------------------
 // Bucket sort
 
@@ -643,7 +699,12 @@ __global__ void k_row_mask(const Geom g, const Item *__restrict__ items,
   const uint32_t nch = chunk_off[g.nbuckets];
   const int ntiles = g.ntu * g.ntv, wk = g.do_w ? g.W : 1;
   const int bw = (g.ngx + 31) / 32;
-  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nch; c += gridDim.x * blockDim.x) {
+  // thread (chunk, plane of the chunk): one chunk's planes in a row took as long as
+  // a dozen dependent atomics
+  const int span = g.S + g.W - 1;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < (uint64_t)nch * span;
+       i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t c = (uint32_t)(i / span);
     const Chunk ch = chunks[c];
     const int slab = (int)(ch.bucket / (uint32_t)ntiles);
     const int tile = (int)(ch.bucket - (uint32_t)slab * ntiles);
@@ -660,13 +721,13 @@ __global__ void k_row_mask(const Geom g, const Item *__restrict__ items,
     const int k_hi =
         min(slab * g.S + (int)((items[ch.end - 1].loc >> 16) & 0xffu) + wk, g.nplanes);
     const int r_lo = tv * g.T, r_hi = tv * g.T + g.T + g.W - 2;  // inclusive
-    for (int k = k_lo; k < k_hi; ++k) {
-      for (int r = r_lo; r <= r_hi + g.T - 1; r += g.T) {
-        int rr = min(r, r_hi);
-        while (rr >= g.ngy) rr -= g.ngy;
-        uint32_t *w = &mask[(int64_t)k * g.ntv + rr / g.T];
-        if ((*w & bits) != bits) atomicOr(w, bits);
-      }
+    const int k = k_lo + (int)(i - (uint64_t)c * span);
+    if (k >= k_hi) continue;
+    for (int r = r_lo; r <= r_hi + g.T - 1; r += g.T) {
+      int rr = min(r, r_hi);
+      while (rr >= g.ngy) rr -= g.ngy;
+      uint32_t *w = &mask[(int64_t)k * g.ntv + rr / g.T];
+      if ((*w & bits) != bits) atomicOr(w, bits);
     }
   }
 }
@@ -765,13 +826,16 @@ static int plane_stats(gb_plan *p, cudaStream_t s) {
   return GB_OK;
 }
 
-// exp(+2 pi i m / n), m < n, rounded from FP64.
-__global__ void k_twiddles(int n, float2 *__restrict__ tw) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+// exp(+2 pi i m / n), m < n, rounded from FP64, for two lengths (the second
+// may be 0).
+__global__ void k_twiddles(int n1, float2 *__restrict__ tw1, int n2, float2 *__restrict__ tw2) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool first = i < n1;
+  const int m = first ? i : i - n1, n = first ? n1 : n2;
   if (m < n) {
     double sn, cs;
     sincospi(2.0 * (double)m / (double)n, &sn, &cs);
-    tw[m] = make_float2((float)cs, (float)sn);
+    (first ? tw1 : tw2)[m] = make_float2((float)cs, (float)sn);
   }
 }
 
@@ -1070,13 +1134,9 @@ static int run_bind(gb_plan *p, cudaStream_t s) {
     GB_LAUNCH_CHECK("k_corr_image");
   }
   if (p->col_fft) {
-    k_twiddles<<<(g.ngy + kThreads - 1) / kThreads, kThreads, 0, s>>>(g.ngy,
-                                                                     p->at<float2>(p->off_twn));
-    GB_LAUNCH_CHECK("k_twiddles");
-  }
-  if (p->row_fft) {
-    k_twiddles<<<(g.ngx + kThreads - 1) / kThreads, kThreads, 0, s>>>(g.ngx,
-                                                                     p->at<float2>(p->off_twx));
+    const int nx = p->row_fft ? g.ngx : 0;
+    k_twiddles<<<(g.ngy + nx + kThreads - 1) / kThreads, kThreads, 0, s>>>(
+        g.ngy, p->at<float2>(p->off_twn), nx, p->at<float2>(p->off_twx));
     GB_LAUNCH_CHECK("k_twiddles");
   }
   if (p->fft64) {
@@ -1087,7 +1147,8 @@ static int run_bind(gb_plan *p, cudaStream_t s) {
     uint32_t *mask = p->at<uint32_t>(p->off_rowmask);
     GB_CUDA(cudaMemsetAsync(mask, 0, 4 * (size_t)g.nplanes * g.ntv, s));
     const unsigned cb = (unsigned)std::min<int64_t>(
-        ((int64_t)p->max_chunks + kThreads - 1) / kThreads, (int64_t)p->num_sms * 16);
+        ((int64_t)p->max_chunks * (g.S + g.W - 1) + kThreads - 1) / kThreads,
+        (int64_t)p->num_sms * 16);
     k_row_mask<Item><<<cb, kThreads, 0, s>>>(g, items, chunks, chunk_off, mask);
     GB_LAUNCH_CHECK("k_row_mask");
     if (prof_on()) {  // host copy for the profiler's byte counts (costs a sync)
@@ -1199,34 +1260,32 @@ int gb_plan_create(const gb_plan_params *params, const double *uvw_dev,
     return GB_ERR_INVALID_ARG;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  // frequencies to the host (validation and the w range)
+  // the w range and the frequencies to the host, in one copy
   std::vector<double> freq(params->nchan);
-  GB_CUDA(cudaMemcpyAsync(freq.data(), freq_dev, 8 * (size_t)params->nchan,
-                          cudaMemcpyDeviceToHost, s));
   double w_lo = 0.0, w_hi = 0.0;
   {
-    const int blocks = 512;
+    const int blocks =
+        (int)std::min<int64_t>((params->nrows + kThreads - 1) / kThreads, 512);
+    const size_t nout = 3 + (size_t)params->nchan;
     double *part = nullptr;
-    GB_CUDA(cudaMallocAsync((void **)&part, 3 * 8 * blocks, s));
+    GB_CUDA(scratch_alloc((void **)&part, 8 * (3 * (size_t)blocks + nout), s));
+    double *out = part + 3 * (size_t)blocks;
     cudaError_t le;
     {
       ProfScope ps(kProfWrange, s, 24.0 * (double)params->nrows);
       k_wrange<<<blocks, kThreads, 0, s>>>(uvw_dev, params->nrows,
                                            params->do_wstacking ? 1 : 0, part);
+      k_wrange_end<<<1, kThreads, 0, s>>>(part, blocks, freq_dev, params->nchan, out);
       le = cudaGetLastError();
     }
-    std::vector<double> hp(3 * blocks);
-    cudaError_t ce = cudaMemcpyAsync(hp.data(), part, 3 * 8 * blocks, cudaMemcpyDeviceToHost, s);
+    std::vector<double> hp(nout);
+    cudaError_t ce = cudaMemcpyAsync(hp.data(), out, 8 * nout, cudaMemcpyDeviceToHost, s);
     cudaFreeAsync(part, s);
     if (le != cudaSuccess) return cuda_fail(le, "k_wrange");
     if (ce != cudaSuccess) return cuda_fail(ce, "w range copy");
     GB_CUDA(cudaStreamSynchronize(s));
-    double rlo = INFINITY, rhi = -INFINITY, bad = 0.0;
-    for (int b = 0; b < blocks; ++b) {
-      rlo = std::fmin(rlo, hp[3 * b]);
-      rhi = std::fmax(rhi, hp[3 * b + 1]);
-      bad += hp[3 * b + 2];
-    }
+    const double rlo = hp[0], rhi = hp[1], bad = hp[2];
+    std::copy(hp.begin() + 3, hp.end(), freq.begin());
     if (bad > 0.0) {
       set_error("uvw holds %.0f rows with non-finite values", bad);
       return GB_ERR_INVALID_ARG;

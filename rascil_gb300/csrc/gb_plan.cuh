@@ -157,6 +157,13 @@ int inv_end(gb_plan *p, void *dirty, int layout, cudaStream_t s);
 int pred_begin(gb_plan *p, const void *dirty, int layout, cudaStream_t s);
 int pred_transform(gb_plan *p, int bi, cudaStream_t s);
 
+// Small device scratch, stream-ordered (free it with cudaFreeAsync on the stream
+// that used it last).  From a memory pool of the library's own, one per device,
+// that keeps at most 32 MiB across synchronisations: the default pool keeps nothing,
+// and an allocation right after a synchronisation took 125 us there.  Safe with
+// any threads and streams, as every stream-ordered allocation.
+cudaError_t scratch_alloc(void **ptr, size_t bytes, cudaStream_t s);
+
 // Let a kernel be launched with any dynamic shared memory the device grants a
 // block.  Never the size of one plan: the opt-in is per kernel, and a plan of
 // smaller tiles made later would lower it under the launches of a larger one.
