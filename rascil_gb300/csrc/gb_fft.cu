@@ -147,24 +147,34 @@ template <int L, int S> __device__ __forceinline__ void dft(float2 *a) {
 // before the barrier.  The caller synchronises before xb is reused.
 // tw[m] = exp(s 2 pi i m / N).
 template <int N, int S>
-__device__ __forceinline__ void col_dft(float2 (&x)[ColShape<N>::M], float2 *__restrict__ xb,
-                                        const float2 *__restrict__ tw, int t, int c,
-                                        float2 (&y)[ColShape<N>::M / ColShape<N>::T]
-                                                   [ColShape<N>::T]) {
+__device__ __forceinline__ void col_dft_in(float2 (&x)[ColShape<N>::M], float2 *__restrict__ xb,
+                                           const float2 *__restrict__ tw, int t, int c) {
   constexpr int T = ColShape<N>::T, M = ColShape<N>::M;
   dft<M, S>(x);
 #pragma unroll
   for (int k1 = 1; k1 < M; ++k1) x[k1] = cmul(x[k1], tw[t * k1]);
 #pragma unroll
   for (int k1 = 0; k1 < M; ++k1) xb[(k1 * T + t) * kCW + c] = x[k1];
+}
+// The second half of it, after the barrier: outputs t + T ii + M k2 in y[k2].
+template <int N, int S>
+__device__ __forceinline__ void col_dft_out(const float2 *__restrict__ xb, int t, int c, int ii,
+                                            float2 (&y)[ColShape<N>::T]) {
+  constexpr int T = ColShape<N>::T;
+#pragma unroll
+  for (int tt = 0; tt < T; ++tt) y[tt] = xb[((t + T * ii) * T + tt) * kCW + c];
+  dft<T, S>(y);
+}
+template <int N, int S>
+__device__ __forceinline__ void col_dft(float2 (&x)[ColShape<N>::M], float2 *__restrict__ xb,
+                                        const float2 *__restrict__ tw, int t, int c,
+                                        float2 (&y)[ColShape<N>::M / ColShape<N>::T]
+                                                   [ColShape<N>::T]) {
+  col_dft_in<N, S>(x, xb, tw, t, c);
   __syncthreads();
 #pragma unroll
-  for (int ii = 0; ii < M / T; ++ii) {
-    const int k1 = t + T * ii;
-#pragma unroll
-    for (int tt = 0; tt < T; ++tt) y[ii][tt] = xb[(k1 * T + tt) * kCW + c];
-    dft<T, S>(y[ii]);
-  }
+  for (int ii = 0; ii < ColShape<N>::M / ColShape<N>::T; ++ii)
+    col_dft_out<N, S>(xb, t, c, ii, y[ii]);
 }
 
 // exp(s 2 pi i m / N), m < N, from the n-point table exp(+2 pi i m / n).
@@ -208,40 +218,92 @@ struct ScreenRot {
 };
 
 // ----------------------------------------------------------------------
-// invert step A: in place, one CTA per (column tile, q2, plane-pol).  HBM
-// bound; without the rows outside the mask 15.2 ms instead of 17.7 (8192 x
-// 4096 columns, 42 planes of 4 pols).
-template <int N1>
-__global__ void __launch_bounds__(ColShape<N1>::THREADS, 3)
-    k_cols_a_inv(const ColGeom cg, const float2 *__restrict__ twn, float2 *__restrict__ grid) {
-  using CS = ColShape<N1>;
-  constexpr int T = CS::T, M = CS::M;
-  extern __shared__ float2 smem[];
-  float2 *xb = smem, *tw = smem + N1 * kCW;
+// The in-place steps: invert step A (A: N = N1, one CTA column per (column
+// tile, q2)) and predict step B (N = N2, per (column tile, k1)).  A CTA runs
+// `per` consecutive plane-pols of the batch through S shared-memory tiles: a
+// warp copies the rows it transforms (rows m T + t of the tile) with 16-byte
+// cp.async S - 1 tiles ahead, and the exchange reuses their slots, so one
+// barrier per tile serves both the exchange and the refill of the tile before.
+// Step A reads only rows in the occupancy mask (the others were never zeroed
+// nor gridded) and takes the rest as zero; step B writes only those rows (no
+// row transform reads the others).
+// HBM bound: two tiles per CTA and as many CTAs as fit keep more bytes in
+// flight than three tiles did, and both more than loads into registers behind
+// one CTA per plane-pol.  8192 x 4096 columns, 42 planes of 4 pols: step A
+// (N = 64) 15.2 ms in registers, 11.8 with three tiles and 4 CTAs, 11.2 with
+// two and 5; step B (N = 128) 11.9, 12.7 with three tiles and 2 CTAs, 10.3
+// with two and 3.
+template <int N> struct ColPipe {
+  static constexpr int S = 2;  // tiles
+  static constexpr int CTAS = N <= 32 ? 8 : N == 64 ? 5 : N == 128 ? 3 : 1;  // per SM
+};
+template <int N, bool A>
+__global__ void __launch_bounds__(ColShape<N>::THREADS, ColPipe<N>::CTAS)
+    k_cols_inplace(const ColGeom cg, const float2 *__restrict__ twn, float2 *__restrict__ grid,
+                   int npp, int per) {
+  using CS = ColShape<N>;
+  constexpr int T = CS::T, M = CS::M, S = ColPipe<N>::S;
+  extern __shared__ __align__(16) float2 smem[];
+  float2 *tw = smem + S * N * kCW;
+  float2 *st = tw + N;  // step A: exp(2 pi i q2 o / n), o < N
   const int c = threadIdx.x % kCW, t = threadIdx.x / kCW;
-  const int p = cg.ox + blockIdx.x * kCW + c;
-  const bool ok = p < cg.ox + cg.nx;
-  const int q2 = blockIdx.y;
-  float2 *plane = grid + (int64_t)blockIdx.z * cg.plane;
-  // rows outside the occupancy mask were never zeroed (nor gridded) and are not read
-  const uint32_t used = cg.rows_used<M>(blockIdx.z, cg.N2 * (t + T * c) + q2, ok);
-  load_twiddles<N1, 1>(tw, twn, cg.n);
-  float2 x[M];
+  const int p0 = cg.ox + blockIdx.x * kCW;
+  const int cols = min(kCW, cg.ox + cg.nx - p0);  // even
+  const int q = blockIdx.y;
+  const int s0 = blockIdx.z * per, ns = min(per, npp - s0);
+  auto row = [&](int r) { return A ? cg.N2 * r + q : N * q + r; };
+  // mask word of lane i's row (i < M): the input t + T i, or output i, of this warp
+  const int mine = A ? row(t + T * c) : q + cg.N1 * (t + T * (c % (M / T)) + M * (c / (M / T)));
+  const uint32_t *word = cg.mask + (int64_t)cg.b0 * cg.ntv + (c < M ? mine / cg.T : 0);
+  auto used = [&](int s) {
+    const uint32_t w = s < ns && c < M ? word[(int64_t)((s0 + s) / cg.NP) * cg.ntv] : 0u;
+    return __ballot_sync(0xffffffffu, w != 0);
+  };
+  const int part = 2 * (c % 16), half = c / 16;  // the lane's columns and row of a copied pair
+  auto load = [&](int s, uint32_t rows) {
+    if (s < ns && part < cols) {
+      const float2 *src = grid + (int64_t)(s0 + s) * cg.plane + p0 + part;
+      float2 *dst = smem + (s % S) * N * kCW + part;
 #pragma unroll
-  for (int m = 0; m < M; ++m)
-    x[m] = used >> m & 1 ? plane[(int64_t)(cg.N2 * (t + T * m) + q2) * cg.ngx + p]
-                         : make_float2(0.f, 0.f);
+      for (int i = 0; i < M / 2; ++i) {
+        const int m = 2 * i + half, r = m * T + t;
+        if (!A || (rows >> m & 1))
+          cp_async16(dst + r * kCW, src + (int64_t)row(r) * cg.ngx);
+        else
+          *reinterpret_cast<float4 *>(dst + r * kCW) = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < S - 1; ++s) load(s, A ? used(s) : 0u);
+  load_twiddles<N, A ? 1 : -1>(tw, twn, cg.n);
+  if (A)
+    for (int o = threadIdx.x; o < N; o += blockDim.x) st[o] = twn[q * o];
   __syncthreads();
-  float2 y[M / T][T];
-  col_dft<N1, 1>(x, xb, tw, t, c, y);
-  if (ok) {
+  for (int s = 0; s < ns; ++s) {
+    const uint32_t rows = used(A ? s + S - 1 : s);
+    float2 *cur = smem + (s % S) * N * kCW;
+    cp_async_wait<S - 2>();
+    __syncwarp();
+    float2 x[M];
 #pragma unroll
-    for (int ii = 0; ii < M / T; ++ii)
+    for (int m = 0; m < M; ++m) x[m] = cur[(m * T + t) * kCW + c];
+    col_dft_in<N, A ? 1 : -1>(x, cur, tw, t, c);
+    __syncthreads();  // exchange complete; tile s - 1 consumed
+    load(s + S - 1, rows);
+    float2 *plane = grid + (int64_t)(s0 + s) * cg.plane + p0 + c;
+#pragma unroll
+    for (int ii = 0; ii < M / T; ++ii) {
+      float2 y[T];
+      col_dft_out<N, A ? 1 : -1>(cur, t, c, ii, y);
 #pragma unroll
       for (int k2 = 0; k2 < T; ++k2) {
         const int o = t + T * ii + M * k2;
-        plane[(int64_t)(cg.N2 * o + q2) * cg.ngx + p] = cmul(y[ii][k2], twn[q2 * o]);
+        if (c < cols && (A || (rows >> (ii + M / T * k2) & 1)))
+          plane[(int64_t)row(o) * cg.ngx] = A ? cmul(y[k2], st[o]) : y[k2];
       }
+    }
   }
 }
 
@@ -438,39 +500,6 @@ __global__ void __launch_bounds__(ColShape<N1>::THREADS, 2)
   }
 }
 
-// predict step B: in place, one CTA per (column tile, k1, plane-pol).  HBM
-// bound; without the rows outside the mask 11.9 ms instead of 14.4 (as above).
-template <int N2>
-__global__ void __launch_bounds__(ColShape<N2>::THREADS, N2 >= 256 ? 1 : 3)
-    k_cols_b_pred(const ColGeom cg, const float2 *__restrict__ twn, float2 *__restrict__ grid) {
-  using CS = ColShape<N2>;
-  constexpr int T = CS::T, M = CS::M;
-  extern __shared__ float2 smem[];
-  float2 *xb = smem, *tw = smem + N2 * kCW;
-  const int c = threadIdx.x % kCW, t = threadIdx.x / kCW;
-  const int p = cg.ox + blockIdx.x * kCW + c;
-  const bool ok = p < cg.ox + cg.nx;
-  const int k1 = blockIdx.y;
-  float2 *plane = grid + (int64_t)blockIdx.z * cg.plane;
-  load_twiddles<N2, -1>(tw, twn, cg.n);
-  float2 x[M];
-#pragma unroll
-  for (int m = 0; m < M; ++m)
-    x[m] = ok ? plane[(int64_t)(cg.N2 * k1 + t + T * m) * cg.ngx + p] : make_float2(0.f, 0.f);
-  // rows outside the occupancy mask are read by no row transform and not written
-  const uint32_t used =
-      cg.rows_used<M>(blockIdx.z, k1 + cg.N1 * (t + T * (c % (M / T)) + M * (c / (M / T))), ok);
-  __syncthreads();
-  float2 y[M / T][T];
-  col_dft<N2, -1>(x, xb, tw, t, c, y);
-#pragma unroll
-  for (int ii = 0; ii < M / T; ++ii)
-#pragma unroll
-    for (int k2 = 0; k2 < T; ++k2)
-      if (used >> (ii + M / T * k2) & 1)
-        plane[(int64_t)(cg.N2 * k1 + t + T * ii + M * k2) * cg.ngx + p] = y[ii][k2];
-}
-
 // ----------------------------------------------------------------------
 // host side
 
@@ -521,6 +550,10 @@ RowPerm row_perm(const gb_plan *p) {
 
 // exchange slots + twiddles
 template <int N> constexpr size_t smem_one() { return sizeof(float2) * ((size_t)N * kCW + N); }
+// tiles + twiddles + step A's outer twiddles
+template <int N> constexpr size_t smem_inplace() {
+  return sizeof(float2) * ((size_t)ColPipe<N>::S * N * kCW + 2 * N);
+}
 // + screen slots and image slots (N/2 inputs per column)
 template <int N, int NP> constexpr size_t smem_a_pred() {
   return smem_one<N>() + sizeof(float2) * N +
@@ -583,7 +616,11 @@ static int setup_np() {
   GB_ATTR((k_cols_b_inv<64, NP>), (smem_b_inv<64, NP>()));
   GB_ATTR((k_cols_b_inv<128, NP>), (smem_b_inv<128, NP>()));
   GB_ATTR((k_cols_b_inv<256, NP>), (smem_b_inv<256, NP>()));
-  GB_ATTR(k_cols_b_pred<256>, smem_one<256>());
+  GB_ATTR((k_cols_inplace<64, true>), smem_inplace<64>());
+  GB_ATTR((k_cols_inplace<128, true>), smem_inplace<128>());
+  GB_ATTR((k_cols_inplace<64, false>), smem_inplace<64>());
+  GB_ATTR((k_cols_inplace<128, false>), smem_inplace<128>());
+  GB_ATTR((k_cols_inplace<256, false>), smem_inplace<256>());
   GB_ATTR((k_cols_a_pred<16, NP>), (smem_a_pred<16, NP>()));
   GB_ATTR((k_cols_a_pred<32, NP>), (smem_a_pred<32, NP>()));
   GB_ATTR((k_cols_a_pred<64, NP>), (smem_a_pred<64, NP>()));
@@ -601,6 +638,32 @@ int setup_col_kernels(gb_plan *p) {
   }
 }
 
+// Invert step A or predict step B of npp plane-pols.  A CTA takes up to 8 of
+// them, fewer where that would leave less than about eight CTAs per SM.
+template <bool A>
+static int run_inplace(gb_plan *p, const ColGeom &cg, const float2 *twn, float2 *grid, int npp,
+                       unsigned tiles, cudaStream_t s) {
+  const int rows = A ? cg.N2 : cg.N1;
+  int per = 8;
+  while (per > 1 && (int64_t)tiles * rows * ((npp + per - 1) / per) < (int64_t)8 * p->num_sms)
+    per /= 2;
+  const dim3 grd(tiles, rows, (npp + per - 1) / per);
+#define GB_COL(N) \
+  k_cols_inplace<N, A><<<grd, ColShape<N>::THREADS, smem_inplace<N>(), s>>>(cg, twn, grid, npp, per)
+  switch (A ? cg.N1 : cg.N2) {
+    case 16: GB_COL(16); break;
+    case 32: GB_COL(32); break;
+    case 64: GB_COL(64); break;
+    case 128: GB_COL(128); break;
+    default:
+      if constexpr (!A) GB_COL(256);
+      break;
+  }
+#undef GB_COL
+  GB_LAUNCH_CHECK("k_cols_inplace");
+  return GB_OK;
+}
+
 template <int NP>
 static int cols_invert_np(gb_plan *p, float2 *grid, int b0, int nb, float *acc, int first,
                           cudaStream_t s) {
@@ -615,17 +678,8 @@ static int cols_invert_np(gb_plan *p, float2 *grid, int b0, int nb, float *acc, 
   const double npix = (double)g.nx * g.ny;
   {
     ProfScope ps(kProfColInvA, s, 2.0 * cols);
-    const dim3 grd(tiles, cg.N2, nb * NP);
-#define GB_COLA(N)                                                                  \
-  k_cols_a_inv<N><<<grd, ColShape<N>::THREADS, smem_one<N>(), s>>>(cg, twn, grid)
-    switch (cg.N1) {
-      case 16: GB_COLA(16); break;
-      case 32: GB_COLA(32); break;
-      case 64: GB_COLA(64); break;
-      default: GB_COLA(128); break;
-    }
-#undef GB_COLA
-    GB_LAUNCH_CHECK("k_cols_a_inv");
+    const int rc = run_inplace<true>(p, cg, twn, grid, nb * NP, tiles, s);
+    if (rc) return rc;
   }
   {
     ProfScope ps(kProfColInvB, s,
@@ -682,18 +736,8 @@ static int cols_predict_np(gb_plan *p, const float *img, int b0, int nb, float2 
   }
   {
     ProfScope ps(kProfColPredB, s, 2.0 * cols);
-    const dim3 grd(tiles, cg.N1, nb * NP);
-#define GB_COLB(N) \
-  k_cols_b_pred<N><<<grd, ColShape<N>::THREADS, smem_one<N>(), s>>>(cg, twn, grid)
-    switch (cg.N2) {
-      case 16: GB_COLB(16); break;
-      case 32: GB_COLB(32); break;
-      case 64: GB_COLB(64); break;
-      case 128: GB_COLB(128); break;
-      default: GB_COLB(256); break;
-    }
-#undef GB_COLB
-    GB_LAUNCH_CHECK("k_cols_b_pred");
+    const int rc = run_inplace<false>(p, cg, twn, grid, nb * NP, tiles, s);
+    if (rc) return rc;
   }
   if (!p->row_fft) {
     // zero the columns outside the image: [0, ox) and [ox + nx, ngx) of every row

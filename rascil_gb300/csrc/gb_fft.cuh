@@ -16,17 +16,8 @@ struct ColGeom {
   int64_t plane;   // ngx * ngy
   int ngx;
   // (plane, row tile) occupancy: invert step A takes rows outside it as zero
-  // without reading them, predict step B does not write them
   const uint32_t *mask;
   int b0, NP, T, ntv;
-  // Bit i < M: row q of lane i of this warp is in the mask of plane-pol pp and
-  // ok holds for this lane.  One word and one division per lane: the same test
-  // row by row in every lane cost the column kernels 60 % of their time.
-  template <int M> __device__ __forceinline__ uint32_t rows_used(int pp, int q, bool ok) const {
-    const int lane = threadIdx.x % 32;
-    const uint32_t w = lane < M ? mask[(int64_t)(b0 + pp / NP) * ntv + q / T] : 0u;
-    return __ballot_sync(0xffffffffu, w != 0) & (ok ? 0xffffffffu : 0u);
-  }
 };
 
 // True when a column of length n has a supported split n = N1 N2
