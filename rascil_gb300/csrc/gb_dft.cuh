@@ -12,8 +12,18 @@ __device__ __forceinline__ float2 cmulc(float2 a, float c, float s) {
   return make_float2(a.x * c - a.y * s, a.x * s + a.y * c);
 }
 __device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// both parts in one packed instruction (a negated operand costs nothing)
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) {
+  return __fadd2_rn(a, make_float2(-b.x, -b.y));
+}
+// a + s i b, a - s i b: two scalar sums, as the packed form would first swap b's parts
+template <int S> __device__ __forceinline__ float2 cadd_si(float2 a, float2 b) {
+  return S > 0 ? make_float2(a.x - b.y, a.y + b.x) : make_float2(a.x + b.y, a.y - b.x);
+}
+template <int S> __device__ __forceinline__ float2 csub_si(float2 a, float2 b) {
+  return cadd_si<-S>(a, b);
+}
 // a * (s i)
 template <int S> __device__ __forceinline__ float2 mul_si(float2 a) {
   return S > 0 ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);

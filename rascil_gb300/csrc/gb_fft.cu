@@ -62,11 +62,11 @@ struct ColShape {
 // In-register L-point DFTs in natural order, z_q = sum_p a_p exp(s 2 pi i p q / L).
 template <int S> __device__ __forceinline__ void dft4(float2 *a) {
   const float2 s02 = cadd(a[0], a[2]), d02 = csub(a[0], a[2]);
-  const float2 s13 = cadd(a[1], a[3]), d13 = mul_si<S>(csub(a[1], a[3]));
+  const float2 s13 = cadd(a[1], a[3]), d13 = csub(a[1], a[3]);
   a[0] = cadd(s02, s13);
   a[2] = csub(s02, s13);
-  a[1] = cadd(d02, d13);
-  a[3] = csub(d02, d13);
+  a[1] = cadd_si<S>(d02, d13);
+  a[3] = csub_si<S>(d02, d13);
 }
 
 template <int S> __device__ __forceinline__ void dft8(float2 *a) {
@@ -74,14 +74,13 @@ template <int S> __device__ __forceinline__ void dft8(float2 *a) {
   float2 o[4] = {a[1], a[3], a[5], a[7]};
   dft4<S>(e);
   dft4<S>(o);
-  const float2 t0 = o[0], t1 = cmulc(o[1], kR2, S * kR2), t2 = mul_si<S>(o[2]),
-               t3 = cmulc(o[3], -kR2, S * kR2);
+  const float2 t0 = o[0], t1 = cmulc(o[1], kR2, S * kR2), t3 = cmulc(o[3], -kR2, S * kR2);
   a[0] = cadd(e[0], t0);
   a[4] = csub(e[0], t0);
   a[1] = cadd(e[1], t1);
   a[5] = csub(e[1], t1);
-  a[2] = cadd(e[2], t2);
-  a[6] = csub(e[2], t2);
+  a[2] = cadd_si<S>(e[2], o[2]);
+  a[6] = csub_si<S>(e[2], o[2]);
   a[3] = cadd(e[3], t3);
   a[7] = csub(e[3], t3);
 }
@@ -415,23 +414,29 @@ __global__ void __launch_bounds__(ColShape<N2>::THREADS, N2 >= 256 ? 1 : 2)
 }
 
 // predict step A from the corrected image: one CTA per (column tile, q2);
-// loops over the batch's planes and the pols.  The image values (inputs
-// m in [M/4, 3M/4) of each thread) and each plane's screens sit in
-// per-thread shared-memory slots; the screens of the batch's later planes
-// come from the first by rotation (ScreenRot).
+// loops over the batch's planes and the pols.  The screens of the CTA's pixels
+// (inputs m in [M/4, 3M/4) of each thread) sit in registers, those of the
+// batch's later planes from the first by rotation (ScreenRot); the image
+// values sit in per-thread shared-memory slots.  Two exchange buffers, so that
+// a tile needs one barrier.
+// Bound by its stores to HBM and, at N = 128, by instructions: with the
+// screens in shared memory, one buffer and 2 CTAs 8.7 ms at 8192 x 4096 columns
+// (N = 64), 42 planes of 4 pols, and 16.4 ms at 16384 x 8192 (N = 128), 14
+// planes; so 7.2 and 15.2.  4 CTAs at N = 64 spill: 7.5.
+template <int N> struct ColPredA {
+  static constexpr int CTAS = N <= 32 ? 6 : N == 64 ? 3 : 2;  // per SM
+};
 template <int N1, int NP>
-__global__ void __launch_bounds__(ColShape<N1>::THREADS, 2)
+__global__ void __launch_bounds__(ColShape<N1>::THREADS, ColPredA<N1>::CTAS)
     k_cols_a_pred(const ColGeom cg, const float2 *__restrict__ twn, const float *__restrict__ img,
                   const ulonglong2 *__restrict__ screen, int do_w, int b0, int nb,
                   float2 *__restrict__ grid) {
   using CS = ColShape<N1>;
   constexpr int T = CS::T, M = CS::M, ML = M / 4, MK = M / 2;
   extern __shared__ float2 smem[];
-  float2 *xb = smem, *tw = smem + N1 * kCW;
-  float2 *st = tw + N1;                                  // exp(-2 pi i q2 o / n), o < N1
-  float2 *scr = st + N1;                                 // [MK][T][kCW] (cos, sin)
-  float2 *rot = scr + MK * T * kCW;                      // [MK][T][kCW] exp(2 pi i D)
-  float *sv = reinterpret_cast<float *>(rot + MK * T * kCW);  // [NP][MK][T][kCW]
+  float2 *tw = smem + 2 * N1 * kCW;
+  float2 *st = tw + N1;                             // exp(-2 pi i q2 o / n), o < N1
+  float *sv = reinterpret_cast<float *>(st + N1);   // [NP][MK][T][kCW]
   const int c = threadIdx.x % kCW, t = threadIdx.x / kCW;
   const int p = cg.ox + blockIdx.x * kCW + c;
   const bool ok = p < cg.ox + cg.nx;
@@ -445,58 +450,51 @@ __global__ void __launch_bounds__(ColShape<N1>::THREADS, 2)
     const int q = cg.N2 * (t + T * (ML + mm)) + q2;
     return (int64_t)(q - cg.oy) * cg.nx + ix;
   };
-  auto slot = [&](int mm) { return (mm * T + t) * kCW + c; };
+  auto slot = [&](int pol, int mm) { return ((pol * MK + mm) * T + t) * kCW + c; };
 #pragma unroll 1
   for (int pol = 0; pol < NP; ++pol)
 #pragma unroll
     for (int mm = 0; mm < MK; ++mm)
-      sv[pol * MK * T * kCW + slot(mm)] = ok ? img[pol * npix + pixel(mm)] : 0.f;
-  __syncthreads();  // twiddles
-  for (int j = 0; j < nb; ++j) {
+      sv[slot(pol, mm)] = ok ? img[pol * npix + pixel(mm)] : 0.f;
+  ScreenRot scr[MK];
 #pragma unroll
-    for (int mm = 0; mm < MK; ++mm) {
-      // plane b0 from the fixed-point phase, later planes by rotation
-      ScreenRot r;
-      if (!(do_w && ok)) {
-        r.unit();
-      } else if (j == 0) {
-        r.start(screen[pixel(mm)], b0);
-        rot[slot(mm)] = make_float2(r.dc, r.ds);
-      } else {
-        const float2 e = scr[slot(mm)], d = rot[slot(mm)];
-        r.cs = e.x;
-        r.sn = e.y;
-        r.dc = d.x;
-        r.ds = d.y;
-        r.next();
-      }
-      scr[slot(mm)] = make_float2(r.cs, r.sn);
-    }
+  for (int mm = 0; mm < MK; ++mm) {
+    if (do_w && ok)
+      scr[mm].start(screen[pixel(mm)], b0);
+    else
+      scr[mm].unit();
+  }
+  __syncthreads();  // twiddles
+  float2 *plane = grid + p;
+  int k = 0;
 #pragma unroll 1
-    for (int pol = 0; pol < NP; ++pol) {
+  for (int j = 0; j < nb; ++j) {
+#pragma unroll 1
+    for (int pol = 0; pol < NP; ++pol, ++k, plane += cg.plane) {
+      float2 *cur = smem + (k & 1) * (N1 * kCW);
       float2 x[M];
 #pragma unroll
       for (int m = 0; m < M; ++m) x[m] = make_float2(0.f, 0.f);
 #pragma unroll
       for (int mm = 0; mm < MK; ++mm) {
-        const float2 e = scr[slot(mm)];
-        const float v = sv[pol * MK * T * kCW + slot(mm)];
-        x[ML + mm] = make_float2(v * e.x, v * e.y);
+        const float v = sv[slot(pol, mm)];
+        x[ML + mm] = make_float2(v * scr[mm].cs, v * scr[mm].sn);
       }
-      float2 y[M / T][T];
-      col_dft<N1, -1>(x, xb, tw, t, c, y);
-      if (ok) {
-        float2 *plane = grid + ((int64_t)j * NP + pol) * cg.plane;
+      col_dft_in<N1, -1>(x, cur, tw, t, c);
+      __syncthreads();
 #pragma unroll
-        for (int ii = 0; ii < M / T; ++ii)
+      for (int ii = 0; ii < M / T; ++ii) {
+        float2 y[T];
+        col_dft_out<N1, -1>(cur, t, c, ii, y);
 #pragma unroll
-          for (int k2 = 0; k2 < T; ++k2) {
-            const int o = t + T * ii + M * k2;
-            plane[(int64_t)(cg.N2 * o + q2) * cg.ngx + p] = cmul(y[ii][k2], st[o]);
-          }
+        for (int k2 = 0; k2 < T; ++k2) {
+          const int o = t + T * ii + M * k2;
+          if (ok) plane[(int64_t)(cg.N2 * o + q2) * cg.ngx] = cmul(y[k2], st[o]);
+        }
       }
-      __syncthreads();  // exchange slots free again
     }
+#pragma unroll
+    for (int mm = 0; mm < MK; ++mm) scr[mm].next();
   }
 }
 
@@ -548,16 +546,14 @@ RowPerm row_perm(const gb_plan *p) {
   return rp;
 }
 
-// exchange slots + twiddles
-template <int N> constexpr size_t smem_one() { return sizeof(float2) * ((size_t)N * kCW + N); }
+
 // tiles + twiddles + step A's outer twiddles
 template <int N> constexpr size_t smem_inplace() {
   return sizeof(float2) * ((size_t)ColPipe<N>::S * N * kCW + 2 * N);
 }
-// + screen slots and image slots (N/2 inputs per column)
+// two exchange buffers + twiddles + image slots (N/2 inputs per column)
 template <int N, int NP> constexpr size_t smem_a_pred() {
-  return smem_one<N>() + sizeof(float2) * N +
-         (2 * sizeof(float2) + sizeof(float) * NP) * (size_t)(N / 2) * kCW;
+  return sizeof(float2) * ((size_t)2 * N * kCW + 2 * N) + sizeof(float) * NP * (size_t)(N / 2) * kCW;
 }
 // two tile buffers + twiddles + accumulator slots (N/2 kept outputs per column)
 template <int N, int NP> constexpr size_t smem_b_inv() {
