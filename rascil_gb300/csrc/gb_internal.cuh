@@ -369,6 +369,13 @@ inline __host__ __device__ constexpr int group_lanes(int W) { return W <= 8 ? 8 
 // values, AW each (zero beyond W), so every group starts on 16 bytes.
 inline __host__ __device__ constexpr int kcache_stride(int AW) { return 4 + 3 * AW; }
 
+// A support of 9 (the FP32 form's at sigma 1.5 and 1.25) leaves 7 of 16 lanes
+// idle: the gridder's sub-grid spread takes three of its rows at a time, 9 lanes
+// each and all pols per lane (LaneRows).  1 / 2 / 4 pols cost 3 / 6 / 12 updates
+// per lane and part where groups of 16 lanes cost 5 / 9 / 18: 222,750 items of 2
+// pols, 1568^2 grid, 57 -> 49 us.
+constexpr int kRowLanes = 9;
+
 struct TileLayout {
   int SW, pitch, plane;
 };
@@ -376,7 +383,12 @@ struct TileLayout {
 inline __host__ __device__ constexpr TileLayout tile_layout(int T, int W, int NP) {
   const int AW = group_lanes(W), G = 32 / AW;
   const int RS = NP >= G ? 1 : G / NP;
-  const int SW = T + W - 1, pitch = congruent_up(SW, AW);
+  const int SW = T + W - 1;
+  if (W == kRowLanes) {  // rows 10 banks apart (an even pitch)
+    const int pitch = congruent_up(SW, kRowLanes + 1);
+    return TileLayout{SW, pitch, SW * pitch};
+  }
+  const int pitch = congruent_up(SW, AW);
   return TileLayout{SW, pitch, congruent_up(SW * pitch, AW * RS)};
 }
 
@@ -393,6 +405,15 @@ struct LaneMap {
     r0 = NP >= G ? 0 : g / NP;
   }
   __device__ __forceinline__ int pol(int i) const { return p0 + i * G; }
+};
+
+template <int NP>
+struct LaneRows {
+  static constexpr int NPL = NP, RS = 3;
+  int a, r0;  // r0 = 3 in the last five lanes: idle
+  __device__ __forceinline__ explicit LaneRows(int lane)
+      : a(lane % kRowLanes), r0(lane / kRowLanes) {}
+  __device__ __forceinline__ int pol(int i) const { return i; }
 };
 
 // Row order of a predict grid after the column transforms: logical row

@@ -178,18 +178,16 @@ __device__ __forceinline__ int kernel_q31(float kv) {
 // w-support on plane k, spread by one warp into the fixed-point sub-grid.
 // WC > 0: the support width as a compile-time constant (no per-row
 // predicate beyond the lane's own); WC = 0: W at run time.
-template <int NP, int AW, int WC, int NU>
-__device__ __forceinline__ void spread_q31_step(const LaneMap<NP, AW> &lm, int W, int k,
-                                                int kbase, int jj0,
+template <int NP, int AW, int WC, int NU, typename LM>
+__device__ __forceinline__ void spread_q31_step(const LM &lm, int W, int k, int kbase, int jj0,
                                                 const float *__restrict__ kc,
                                                 const float2 *__restrict__ cc, int *acc,
                                                 const TileLayout &L) {
-  using LM = LaneMap<NP, AW>;
   constexpr int KS = kcache_stride(AW);
   constexpr int WM = WC > 0 ? WC : AW;                  // rows bound, compile time
   constexpr int NR = (WM + LM::RS - 1) / LM::RS;        // support rows per lane (at most)
   constexpr int NK = LM::RS == 1 ? (WM + 3) / 4 * 4 : 1;  // Q31 row values held
-  const bool lane_in = lm.a < W;
+  const bool lane_in = lm.a < W && lm.r0 < LM::RS;
   const int im_off = NP * L.plane;
   int kq[NU][NK];
   int cre[NU][LM::NPL], cim[NU][LM::NPL];
@@ -246,9 +244,9 @@ __device__ __forceinline__ void spread_q31_step(const LaneMap<NP, AW> &lm, int W
 // w-support on k): warp w takes items jj_lo + w + 2 kWarps i and the items
 // kWarps after them, two per step (independent chains of atomics), and a
 // last odd item alone.
-template <int NP, int AW, int WC>
-__device__ __forceinline__ void spread_q31(const LaneMap<NP, AW> &lm, int warp, int W, int k,
-                                           int kbase, int jj_lo, int jj_hi,
+template <int NP, int AW, int WC, typename LM>
+__device__ __forceinline__ void spread_q31(const LM &lm, int warp, int W, int k, int kbase,
+                                           int jj_lo, int jj_hi,
                                            const float *__restrict__ kc,
                                            const float2 *__restrict__ cc, int *acc,
                                            const TileLayout &L) {
@@ -274,8 +272,9 @@ __device__ __forceinline__ void spread_fixed(const LaneMap<NP, AW> &lm, int warp
     spread_q31<NP, AW, AW == 8 ? 7 : 0>(lm, warp, W, k, kbase, jj_lo, jj_hi, kc, cc, acc, L32);
   } else if (AW == 8 && W == 7) {
     spread_q31<NP, AW, AW == 8 ? 7 : 0>(lm, warp, W, k, kbase, jj_lo, jj_hi, kc, cc, acc, L);
-  } else if (AW == 16 && W == 9) {
-    spread_q31<NP, AW, AW == 16 ? 9 : 0>(lm, warp, W, k, kbase, jj_lo, jj_hi, kc, cc, acc, L);
+  } else if (AW == 16 && W == kRowLanes) {
+    spread_q31<NP, AW, AW == 16 ? kRowLanes : 0>(LaneRows<NP>(threadIdx.x & 31), warp, W, k,
+                                                 kbase, jj_lo, jj_hi, kc, cc, acc, L);
   } else {
     spread_q31<NP, AW, 0>(lm, warp, W, k, kbase, jj_lo, jj_hi, kc, cc, acc, L);
   }
