@@ -316,7 +316,10 @@ __device__ __forceinline__ void grid_chunk(
     const int lk_last = (int)((items[ch.end - 1].loc >> 16) & 0xffu);
     const int k_lo = max(kbase + lk_first, b0);
     const int k_hi = min(min(kbase + lk_last + W, g.nplanes), b0 + nb);
-    if (k_lo >= k_hi) return;  // (block-uniform) no item reaches this batch's planes
+    if (k_lo >= k_hi) {  // (block-uniform) no item reaches this batch's planes
+      __syncthreads();   // the work index is read by every thread before it changes
+      return;
+    }
     const int n = (int)(ch.end - ch.begin);
     const bool direct = n * W * W < SW2;
     // chunk scale for the fixed-point sub-grid: 2^30 / sum_j max |component|,
