@@ -28,7 +28,7 @@ constexpr double kSpeedOfLight = 299792458.0;  // rascil/phyconst.py:6
 constexpr int kThreads = 256;                   // block size of the tile kernels
 constexpr int kWarps = kThreads / 32;
 constexpr int kChunkItems = 256;                // items per work chunk (FP32 form)
-constexpr int kChunkItems64 = 64;               // and in the FP64 form
+constexpr int kChunkItems64 = 64;               // and in the FP64 form, at most
 constexpr int kMaxSupport = 16;
 constexpr int kMaxQuad = 48;                    // Gauss-Legendre nodes (half interval)
 constexpr int kMaxSlab = 128;                   // w-planes per bucket slab

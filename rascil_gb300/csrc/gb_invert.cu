@@ -487,7 +487,7 @@ template <int NP, int AW>
 __global__ void __launch_bounds__(kThreads)
     k_grid(const Geom g, const ItemF *__restrict__ items, const float2 *__restrict__ cvis,
            const Chunk *__restrict__ chunks, const uint32_t *__restrict__ chunk_off, int b0, int nb,
-           float2 *__restrict__ grid, uint32_t *__restrict__ counter) {
+           float2 *__restrict__ grid, uint32_t *__restrict__ counter, int part) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int *acc = reinterpret_cast<int *>(smem_raw);  // [re pols | im pols][SW][pitch]
   const TileLayout L = tile_layout(g.T, g.W, NP);
@@ -504,12 +504,18 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ float s_scale[2];
   __shared__ int s_first[kMaxSlab + 1];
   for (;;) {
-    if (threadIdx.x == 0) s_ci = c_begin + atomicAdd(counter, 1u);
+    if (threadIdx.x == 0) s_ci = atomicAdd(counter, 1u);
     __syncthreads();
-    const uint32_t ci = s_ci;
+    // ticket: a chunk and which `part` of its items
+    const uint32_t split = (uint32_t)(kChunkItems / part), ci = c_begin + s_ci / split;
     if (ci >= c_end) break;
-    grid_chunk<NP, AW>(g, items, cvis, chunks[ci], b0, nb, grid, acc, kc, cc, s_red, s_scale,
-                          s_first);
+    Chunk ch = chunks[ci];
+    ch.begin += s_ci % split * (uint32_t)part;
+    ch.end = min(ch.end, ch.begin + (uint32_t)part);
+    if (ch.begin < ch.end)
+      grid_chunk<NP, AW>(g, items, cvis, ch, b0, nb, grid, acc, kc, cc, s_red, s_scale, s_first);
+    else
+      __syncthreads();  // s_ci read by every thread
   }
 }
 
@@ -620,6 +626,16 @@ size_t grid_smem_bytes(const gb_plan *p) {
              (kcache_stride(group_lanes(p->g.W)) * sizeof(float) + p->g.NP * sizeof(float2));
 }
 
+// Items that a CTA of k_grid takes at a time: a chunk's 256, or with few items a
+// half or a quarter of them, so that there are 512 parts to spread over the chip
+// (a part runs through its planes one after the other).  Whole inverts: 24,192 items
+// of 1 pol 111 -> 94 us, 22,176 of 4 pols 213 -> 196; parts of 32 gained less.
+static int grid_part(const Geom &g) {
+  int part = kChunkItems;
+  while (part > 64 && g.nitems < 512u * (uint32_t)part) part /= 2;
+  return part;
+}
+
 // The invert driver in steps (a batch of plans interleaves them across
 // plans: gb_batch.cu).  begin: per-item values; per w-plane batch bi: zero,
 // grid, transform (+ screen and accumulation); end: correction and layout.
@@ -636,11 +652,13 @@ static int inv_begin_impl(gb_plan *p, const void *vis, int npv, const void *wgt,
   const Item *items = p->at<Item>(p->off_items);
   GB_CUDA(cudaMemsetAsync(counters, 0, 4 * (size_t)p->nbatches, s));
   if (sumwt) GB_CUDA(cudaMemsetAsync(sumwt, 0, sizeof(double) * NP, s));
-  // two items per thread: half the blocks, and with them half the sums of weights
-  // that meet in one word (222,750 items: 13.3 us with one item, 10.3 with two,
-  // 13.8 with four, where too few threads are left to hide the gathers)
+  // one item per thread up to two blocks per SM, then two: half the blocks, and
+  // with them half the sums of weights that meet in one word (222,750 items: 13.3 us
+  // with one item, 10.3 with two, 13.8 with four, where too few threads are left to
+  // hide the gathers; 36,180 items of 4 pols: 7.6 with one, 10.7 with two)
+  const int64_t one = ((int64_t)g.nitems + kThreads - 1) / kThreads;
   const unsigned item_blocks = (unsigned)std::min<int64_t>(
-      ((int64_t)g.nitems + 2 * kThreads - 1) / (2 * kThreads), (int64_t)p->num_sms * 16);
+      std::min<int64_t>(one, std::max<int64_t>((one + 1) / 2, p->num_sms * 2)), p->num_sms * 16);
   const double fb = ftype == GB_FLAGS_I64 ? 8.0 : (ftype == GB_FLAGS_U8 ? 1.0 : 0.0);
   const double per = sizeof(Item) + (psf ? 0.0 : npv * sizeof(C)) +
                      (wgt ? NP * sizeof(R) : 0.0) + npv * fb + NP * sizeof(C);
@@ -706,12 +724,13 @@ static int inv_grid_impl(gb_plan *p, int bi, cudaStream_t s) {
     const Chunk *chunks = p->at<Chunk>(p->off_chunks);
     const uint32_t *chunk_off = p->at<uint32_t>(p->off_chunk_off);
     const size_t smem = grid_smem_bytes(p);
+    const int part = grid_part(g);
     if (group_lanes(g.W) == 8)
       k_grid<NP, 8><<<p->grid_blocks, kThreads, smem, s>>>(g, items, cvis, chunks, chunk_off, b0,
-                                                           nb, grid, counters + bi);
+                                                           nb, grid, counters + bi, part);
     else
       k_grid<NP, 16><<<p->grid_blocks, kThreads, smem, s>>>(g, items, cvis, chunks, chunk_off, b0,
-                                                            nb, grid, counters + bi);
+                                                            nb, grid, counters + bi, part);
     GB_LAUNCH_CHECK("k_grid");
     return GB_OK;
   }
