@@ -383,8 +383,8 @@ def _ncu_traffic(kernel):
 
 # update-rate rooflines: shared-memory instructions per (item, pol, cell) update
 UPDATE_COST = {"k_grid": ("atomics", 2.0, "2 conflict-free 32-bit shared atomic adds (re, im)"),
-               "k_degrid": ("loads", 1.0, "1 8-byte grid read (complex64) through the L1 data "
-                                         "pipe, against that pipe's conflict-free 8-byte "
+               "k_degrid": ("loads", 1.0, "1 8-byte grid read (complex64) from a staged "
+                                         "window, against the conflict-free 8-byte "
                                          "shared-load rate")}
 
 
@@ -1160,7 +1160,9 @@ def bench_autograd(args):
     gt = torch.from_numpy(g_true).to(device)
     obs = apply_gains(v_true, gt, a1, a2).to(torch.complex64).contiguous()
     del v_true
+    _lib.profile_enable(True)  # the plan keeps its occupancy for the byte counts
     plan = Plan(fu, f, npix, npix, cell, cell, eps, True, npol=1, precision="fp32")
+    _lib.profile_enable(False)
     # image step 1 / L: L = 2 lambda_max(A^H A) (power iteration through the
     # plan's own predict and adjoint) with a margin for gains near 1
     with torch.no_grad():
@@ -1576,14 +1578,14 @@ def workload_config(wl):
 
 # What bounds each kernel of the step (ncu summaries under profiles/).
 KERNEL_BOUND = {
-    "k_grid": "shared-memory pipe (atomics and the sub-grid flush) and instruction issue "
-              "(update rate in roofline.secondary)",
-    "k_degrid": "L1 data pipe: grid rows read through L1, plus the item cache in shared memory "
+    "k_grid": "integer multiplies, the shared-memory pipe (atomics and the sub-grid flush) and "
+              "instruction issue (update rate in roofline.secondary)",
+    "k_degrid": "shared memory: windows of the grid staged per chunk, 16 warps per SM "
                 "(update rate in roofline.secondary)",
-    "k_rows_forward": "instruction issue (DRAM traffic = algorithmic bytes)",
-    "k_rows_inverse": "instruction issue (DRAM traffic = algorithmic bytes)",
+    "k_rows_forward": "instruction issue and the latency of the exchanges",
+    "k_rows_inverse": "instruction issue and the latency of the exchanges",
     "k_col_a_inv": "hbm", "k_col_b_inv": "hbm", "k_col_b_pred": "hbm",
-    "k_col_a_pred": "hbm", "grid_zero": "hbm (write only)",
+    "k_col_a_pred": "instruction issue and hbm (write only)", "grid_zero": "hbm (write only)",
 }
 
 

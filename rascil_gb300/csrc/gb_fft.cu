@@ -673,7 +673,7 @@ static int cols_invert_np(gb_plan *p, float2 *grid, int b0, int nb, float *acc, 
   const double cols = (double)nb * NP * cg.n * g.nx * sizeof(float2);  // image columns
   const double npix = (double)g.nx * g.ny;
   {
-    ProfScope ps(kProfColInvA, s, 2.0 * cols);
+    ProfScope ps(kProfColInvA, s, (p->used_rows(b0, nb) + 1.0) * cols);  // used rows in, all out
     const int rc = run_inplace<true>(p, cg, twn, grid, nb * NP, tiles, s);
     if (rc) return rc;
   }
@@ -731,7 +731,7 @@ static int cols_predict_np(gb_plan *p, const float *img, int b0, int nb, float2 
     GB_LAUNCH_CHECK("k_cols_a_pred");
   }
   {
-    ProfScope ps(kProfColPredB, s, 2.0 * cols);
+    ProfScope ps(kProfColPredB, s, (1.0 + p->used_rows(b0, nb)) * cols);  // all in, used rows out
     const int rc = run_inplace<false>(p, cg, twn, grid, nb * NP, tiles, s);
     if (rc) return rc;
   }
