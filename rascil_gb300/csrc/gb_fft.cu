@@ -224,8 +224,8 @@ struct ScreenRot {
 // cp.async S - 1 tiles ahead, and the exchange reuses their slots, so one
 // barrier per tile serves both the exchange and the refill of the tile before.
 // Step A reads only rows in the occupancy mask (the others were never zeroed
-// nor gridded) and takes the rest as zero; step B writes only those rows (no
-// row transform reads the others).
+// nor gridded) and takes the rest as zero; step B writes only those rows (the
+// others' transforms are never degridded).
 // HBM bound: two tiles per CTA and as many CTAs as fit keep more bytes in
 // flight than three tiles did, and both more than loads into registers behind
 // one CTA per plane-pol.  8192 x 4096 columns, 42 planes of 4 pols: step A
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(ColShape<N>::THREADS, ColPipe<N>::CTAS)
                    int npp, int per) {
   using CS = ColShape<N>;
   constexpr int T = CS::T, M = CS::M, S = ColPipe<N>::S;
-  extern __shared__ __align__(16) float2 smem[];
+  extern __shared__ __align__(128) float2 smem[];
   float2 *tw = smem + S * N * kCW;
   float2 *st = tw + N;  // step A: exp(2 pi i q2 o / n), o < N
   const int c = threadIdx.x % kCW, t = threadIdx.x / kCW;

@@ -5,16 +5,19 @@
 //                           w-centring rotation; sum the weights per pol.
 // Per batch of w-planes:
 //             k_grid        (FP32 form; the FP64 form's is k_grid64, gb_fp64.cu)
-//                           one CTA per work chunk (<= 256 items of one
-//                           (slab, tile) bucket): the tile's sub-grid lives in
-//                           shared memory, each warp spreads one item at a
-//                           time over its W x W support (kernel values per
-//                           support row/column, exchanged by warp shuffles),
-//                           then the sub-grid is flushed to the HBM grid with
-//                           vector atomics.  Sparse chunks skip the sub-grid.
-//             cuFFT         2-D c2c, e^{+2 pi i}, batched over planes x pols
-//             k_screen_acc  reads the central block of each plane, applies the
-//                           w-screen exp(-2 pi i w_k (n-1-tc)) and accumulates.
+//                           one CTA per work chunk or part of one (<= 256 items
+//                           of one (slab, tile) bucket): the tile's sub-grid and
+//                           the items' kernel values live in shared memory, each
+//                           warp spreads two items at a time over their W x W
+//                           supports, then the sub-grid is flushed to the HBM
+//                           grid with vector atomics.  Sparse chunks skip the
+//                           sub-grid.
+//             transforms    rows and columns with screens and accumulation
+//                           (gb_rows.cu, gb_fft.cu), k_fft64 (gb_fft64.cu) or
+//                           cuFFT 2-D c2c, e^{+2 pi i}
+//             k_screen_acc  (with k_fft64 and cuFFT) reads the central block of each
+//                           plane, applies the w-screen exp(-2 pi i w_k (n-1-tc))
+//                           and accumulates; without w-stacking left to k_finalize.
 // Once:       k_finalize    multiply by the correction image, write the
 //                           requested layout.
 #include <cufft.h>
