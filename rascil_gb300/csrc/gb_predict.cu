@@ -803,10 +803,10 @@ static size_t degrid_staged_smem(const Geom &g) {
 // The staged degridder's tiles: supports of up to 7 cells (four cell pairs a
 // row), even tile sides (16-byte copies) no wider than the grid, two windows in an
 // SM's shared memory (32-cell tiles and smaller).  Others, supports of 8 to 16
-// cells, and plans without w-stacking take the warp degridder: on one plane a
-// staged window serves 1, 2 or 4 of the 8 lanes of an item (6.7M items, 256^2 to
-// 4096^2 pixels: 0.78-1.21 ms by warps, 1.10-1.71 staged at 1 pol; 1.29-2.93 and
-// 1.56-3.16 at 4).
+// cells, and plans without w-stacking take the warp degridder: a window of one
+// plane holds 1, 2 or 4 of the 8 sheets that share an item's weights and its
+// reduction (6.7M items, 256^2 to 4096^2 pixels: 0.78-1.21 ms by warps, 1.10-1.71
+// staged at 1 pol; 1.29-2.93 and 1.56-3.16 at 4).
 static int degrid_width(const Geom &g) {
   const int SW = g.T + g.W - 1;
   const bool staged = g.do_w && g.W <= kStageMaxW && g.T % 2 == 0 && SW + 1 <= g.ngx &&
