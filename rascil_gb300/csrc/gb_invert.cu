@@ -486,7 +486,9 @@ __device__ __forceinline__ void grid_chunk(
   }
 }
 
-template <int NP, int AW>
+// SPLIT: tickets are `part` items of a chunk (grid_part).  Two instances, as the
+// whole-chunk loop with run-time parts cost 6 % on large problems (33.0 -> 35.1 ms).
+template <int NP, int AW, bool SPLIT>
 __global__ void __launch_bounds__(kThreads)
     k_grid(const Geom g, const ItemF *__restrict__ items, const float2 *__restrict__ cvis,
            const Chunk *__restrict__ chunks, const uint32_t *__restrict__ chunk_off, int b0, int nb,
@@ -507,18 +509,24 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ float s_scale[2];
   __shared__ int s_first[kMaxSlab + 1];
   for (;;) {
-    if (threadIdx.x == 0) s_ci = atomicAdd(counter, 1u);
+    if (threadIdx.x == 0) s_ci = SPLIT ? atomicAdd(counter, 1u) : c_begin + atomicAdd(counter, 1u);
     __syncthreads();
-    // ticket: a chunk and which `part` of its items
-    const uint32_t split = (uint32_t)(kChunkItems / part), ci = c_begin + s_ci / split;
-    if (ci >= c_end) break;
-    Chunk ch = chunks[ci];
-    ch.begin += s_ci % split * (uint32_t)part;
-    ch.end = min(ch.end, ch.begin + (uint32_t)part);
-    if (ch.begin < ch.end)
-      grid_chunk<NP, AW>(g, items, cvis, ch, b0, nb, grid, acc, kc, cc, s_red, s_scale, s_first);
-    else
-      __syncthreads();  // s_ci read by every thread
+    if constexpr (SPLIT) {
+      const uint32_t split = (uint32_t)(kChunkItems / part), ci = c_begin + s_ci / split;
+      if (ci >= c_end) break;
+      Chunk ch = chunks[ci];
+      ch.begin += s_ci % split * (uint32_t)part;
+      ch.end = min(ch.end, ch.begin + (uint32_t)part);
+      if (ch.begin < ch.end)
+        grid_chunk<NP, AW>(g, items, cvis, ch, b0, nb, grid, acc, kc, cc, s_red, s_scale, s_first);
+      else
+        __syncthreads();  // s_ci read by every thread
+    } else {
+      const uint32_t ci = s_ci;
+      if (ci >= c_end) break;
+      grid_chunk<NP, AW>(g, items, cvis, chunks[ci], b0, nb, grid, acc, kc, cc, s_red, s_scale,
+                         s_first);
+    }
   }
 }
 
@@ -728,12 +736,15 @@ static int inv_grid_impl(gb_plan *p, int bi, cudaStream_t s) {
     const uint32_t *chunk_off = p->at<uint32_t>(p->off_chunk_off);
     const size_t smem = grid_smem_bytes(p);
     const int part = grid_part(g);
-    if (group_lanes(g.W) == 8)
-      k_grid<NP, 8><<<p->grid_blocks, kThreads, smem, s>>>(g, items, cvis, chunks, chunk_off, b0,
-                                                           nb, grid, counters + bi, part);
-    else
-      k_grid<NP, 16><<<p->grid_blocks, kThreads, smem, s>>>(g, items, cvis, chunks, chunk_off, b0,
-                                                            nb, grid, counters + bi, part);
+#define GB_GRID(AW, SPLIT)                                                                     \
+  k_grid<NP, AW, SPLIT><<<p->grid_blocks, kThreads, smem, s>>>(                                \
+      g, items, cvis, chunks, chunk_off, b0, nb, grid, counters + bi, part)
+    if (group_lanes(g.W) == 8) {
+      if (part < kChunkItems) GB_GRID(8, true); else GB_GRID(8, false);
+    } else {
+      if (part < kChunkItems) GB_GRID(16, true); else GB_GRID(16, false);
+    }
+#undef GB_GRID
     GB_LAUNCH_CHECK("k_grid");
     return GB_OK;
   }
@@ -1001,10 +1012,10 @@ int run_ms2dirty(gb_plan *p, const void *vis, int npv, const void *wgt, const vo
 #undef GB_CASE
 }
 
-template <int NP, int AW>
-static int setup_grid_aw(gb_plan *p) {
+template <int NP, int AW, bool SPLIT>
+static int setup_grid_split(gb_plan *p) {
   const size_t smem = grid_smem_bytes(p);
-  auto k = k_grid<NP, AW>;
+  auto k = k_grid<NP, AW, SPLIT>;
   const int rc = allow_shared_memory(k);
   if (rc) return rc;
   int per_sm = 0;
@@ -1015,6 +1026,12 @@ static int setup_grid_aw(gb_plan *p) {
   }
   p->grid_blocks = per_sm * p->num_sms;
   return GB_OK;
+}
+
+template <int NP, int AW>
+static int setup_grid_aw(gb_plan *p) {
+  return grid_part(p->g) < kChunkItems ? setup_grid_split<NP, AW, true>(p)
+                                       : setup_grid_split<NP, AW, false>(p);
 }
 
 template <int NP>
