@@ -260,12 +260,13 @@ __global__ void __launch_bounds__(kThreads)
   constexpr int kParts = kChunkItems64 / 32;
   uint32_t c_begin, c_end;
   batch_chunks(g, chunk_off, b0, nb, c_begin, c_end);
-  // this lane's support cells: (b << 8) | a, or -1 beyond W x W
+  // this lane's support cells: (b << 8) | a.  Beyond W x W the last cell, at weight
+  // 0: only cells of a support are sure to be written (0 times a NaN is a NaN)
   int ab[NI];
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
-    const int cell = lane + 32 * i, b = cell / W;
-    ab[i] = b < W ? ((b << 8) | (cell - b * W)) : -1;
+    const int cell = min(lane + 32 * i, W * W - 1), b = cell / W;
+    ab[i] = (b << 8) | (cell - b * W);
   }
   for (;;) {
     uint32_t u = 0;
@@ -307,18 +308,14 @@ __global__ void __launch_bounds__(kThreads)
         int64_t off[NI];
 #pragma unroll
         for (int i = 0; i < NI; ++i) {
-          w[i] = 0.0;
-          off[i] = 0;
-          if (ab[i] >= 0) {
-            const int a = ab[i] & 0xff, b = ab[i] >> 8;
-            int p = tu * T + lu + a;
-            while (p >= g.ngx) p -= g.ngx;
-            int q = tv * T + lv + b;
-            while (q >= g.ngy) q -= g.ngy;
-            const double k2 = kj[a] * kj[W + b];
-            w[i] = ((p + q) & 1) ? -k2 : k2;
-            off[i] = (int64_t)rp.row(q) * g.ngx + p;
-          }
+          const int a = ab[i] & 0xff, b = ab[i] >> 8;
+          int p = tu * T + lu + a;
+          while (p >= g.ngx) p -= g.ngx;
+          int q = tv * T + lv + b;
+          while (q >= g.ngy) q -= g.ngy;
+          const double k2 = lane + 32 * i < W * W ? kj[a] * kj[W + b] : 0.0;
+          w[i] = ((p + q) & 1) ? -k2 : k2;
+          off[i] = (int64_t)rp.row(q) * g.ngx + p;
         }
         double ar[NP], ai[NP];
 #pragma unroll
