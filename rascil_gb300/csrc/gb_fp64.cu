@@ -168,10 +168,14 @@ __global__ void __launch_bounds__(kThreads)
     const int bw = s_box[1] - x_lo + W, bh = s_box[3] - y_lo + W;
     const uint32_t bad = S <= DBL_MAX ? s_bad : 0xfu;
     if (threadIdx.x == 0 && bad) {
-      for (int p = 0; p < NP; ++p)
-        if (bad >> p & 1u)
-          atomicAdd(&grid[(size_t)(k_lo - b0) * NP * plane + p * plane].x,
-                    __longlong_as_double(0x7ff8000000000000LL));
+      // a cell of the chunk's own: the transforms read no bin that no item reaches
+      int p = tu * T + x_lo, q = tv * T + y_lo;
+      while (p >= g.ngx) p -= g.ngx;
+      while (q >= g.ngy) q -= g.ngy;
+      double2 *cell = grid + (size_t)(k_lo - b0) * NP * plane + (size_t)q * g.ngx + p;
+      for (int pol = 0; pol < NP; ++pol)
+        if (bad >> pol & 1u)
+          atomicAdd(&cell[pol * plane].x, __longlong_as_double(0x7ff8000000000000LL));
     }
     __syncthreads();
     for (int k = k_lo; k < k_hi; ++k) {

@@ -94,3 +94,29 @@ def test_results_do_not_depend_on_the_buffer(precision, transform, nx, ny, npol,
         bad = numpy.count_nonzero(~numpy.isfinite(stale))
         assert bad == 0, "%d of %d values not finite" % (bad, stale.size)
         assert rel_rms(stale, clean) < tol
+
+
+@pytest.mark.parametrize("nx,ny,eps,kw", [
+    (256, 256, 1e-12, {}), (512, 128, 1e-10, dict(planes_per_batch=4)),
+    (486, 250, 1e-11, {}), (64, 64, 1e-3, dict(sigma=2.0, tile=4)),
+])
+@pytest.mark.parametrize("bad", [numpy.nan, numpy.inf])
+def test_non_finite_values_through_own_transforms(nx, ny, eps, kw, bad):
+    """A non-finite visibility makes its polarisation's whole image non-finite
+    also where no visibility reaches the grid's first cells, and leaves nothing
+    behind: predictions of the same plan stay as they were."""
+    from rascil_gb300 import wgridder
+    pixsize = 2e-4
+    uvw, freq, ms, img = _problem(nx, ny, 2, pixsize, True)
+    plan = wgridder.Plan(uvw, freq, nx, ny, pixsize, pixsize, eps, True, npol=2,
+                         precision="fp64", **kw)
+    _check_transform(plan.info, FP64_OWN, nx, ny)
+    before = plan.dirty2ms(img).cpu().numpy()
+    clean = plan.ms2dirty(ms).cpu().numpy()
+    ms[317, 1, 1] = bad
+    dirty = plan.ms2dirty(ms).cpu().numpy()
+    after = plan.dirty2ms(img).cpu().numpy()
+    plan.close()
+    assert not numpy.isfinite(dirty[1]).any()
+    assert rel_rms(dirty[0], clean[0]) < 1e-13
+    assert numpy.isfinite(after).all() and rel_rms(after, before) < 1e-13
