@@ -103,16 +103,6 @@ __global__ void __launch_bounds__(kThreads)
 // (16 cycles of the SM's FP64 pipe each) where sincospi with its argument
 // reduction takes about 30.  m comes out of the low bits of d S + 1.5 2^52
 // (|d S| < 2^50).
-constexpr int kTurnTable = 256;
-
-__device__ __forceinline__ void turn_table(double2 *tab) {
-  for (int i = threadIdx.x; i < kTurnTable; i += blockDim.x) {
-    double s, c;
-    sincospi(2.0 * i / kTurnTable, &s, &c);
-    tab[i] = make_double2(c, s);
-  }
-}
-
 // S = kTurnTable f / c as a double and what that leaves out; f = f_hi + f_lo.
 struct TurnScale {
   double hi, lo;

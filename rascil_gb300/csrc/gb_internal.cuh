@@ -308,43 +308,82 @@ struct PlaneTurns {
     const unsigned long long ph = a + (unsigned long long)(unsigned)j * d;
     return (float)(int)(unsigned)(ph >> 32) * 0x1p-32f;
   }
-  __device__ __forceinline__ double turns_f64(int j) const {
-    const unsigned long long ph = a + (unsigned long long)(unsigned)j * d;
-    return (double)(long long)ph * 0x1p-64;
-  }
-  __device__ __forceinline__ float turns(int j, float) const { return turns_f32(j); }
-  __device__ __forceinline__ double turns(int j, double) const { return turns_f64(j); }
 };
 
-// The w-screens exp(2 pi i turns) of planes b0, b0 + 1, ... at one pixel, in
-// order.  FP32: a sincos of each plane's phase.  FP64: exact every eighth plane
-// (35 FP64 instructions), rotated by the plane step in between (4; an error of
-// a rounding per step).
+// exp(2 pi i m / kTurnTable), m < kTurnTable, by the whole block into shared memory
+// (complete after the caller's barrier): the first octant by sincospi, one warp's
+// worth, the rest its mirrors (256 sincospi a block would be 5120 cycles of the
+// SM's FP64 pipe).
+constexpr int kTurnTable = 256;
+
+__device__ __forceinline__ void turn_table(double2 *tab) {
+  constexpr int Q = kTurnTable / 4, O = Q / 2;
+  for (int m = threadIdx.x; m < O; m += blockDim.x)
+    sincospi(2.0 * m / kTurnTable, &tab[m].y, &tab[m].x);
+  if (threadIdx.x == 0) tab[O] = make_double2(0.70710678118654752440, 0.70710678118654752440);
+  __syncthreads();
+  for (int i = threadIdx.x; i < kTurnTable; i += blockDim.x) {
+    if (i <= O) continue;
+    const int m = i % Q;
+    double2 v = tab[m > O ? Q - m : m];
+    if (m > O) v = make_double2(v.y, v.x);
+    const int q = i / Q;  // times i^q
+    if (q & 1) v = make_double2(-v.y, v.x);
+    if (q & 2) v = make_double2(-v.x, -v.y);
+    tab[i] = v;
+  }
+}
+
+// The w-screens exp(2 pi i turns) of planes b0, b0 + 1, ... at one pixel.
+// FP32: a sincos of each plane's phase.  FP64: the phase's nearest point of a
+// turn_table, turned on by the rest r, |r| <= pi / 256 (Taylor, the first terms
+// left out below 1e-17), and only that small turn's part added to the table's
+// value, so two roundings are all there is: 5.2e-17 rms against 128-bit arithmetic
+// (8.5e-17 by sincospi, as the phase is first rounded to a double).  15 FP64
+// instructions a plane against sincospi's 35.  (Turning seven planes of eight on
+// from the one before takes 4, but its error is 3.6e-16 rms: a predict of 520,192
+// items and 20 planes of 1024^2 pixels 8.97 ms with that, 9.25 like this.)
 template <typename R> struct PlaneScreen {
   PlaneTurns pt;
   R c, s;
+  __device__ __forceinline__ explicit PlaneScreen(const double2 *) {}
   __device__ __forceinline__ void start(const Geom &g, int b0, double tprime) {
     pt.start(g, b0, tprime);
   }
-  __device__ __forceinline__ void plane(int j) { sincos_2pi(pt.turns(j, (R)0), &s, &c); }
+  __device__ __forceinline__ void plane(int j) { sincos_2pi(pt.turns_f32(j), &s, &c); }
 };
 template <> struct PlaneScreen<double> {
   PlaneTurns pt;
-  double c, s, dc, ds;
+  const double2 *tab;
+  double c, s;
+  __device__ __forceinline__ explicit PlaneScreen(const double2 *t) : tab(t) {}
   __device__ __forceinline__ void start(const Geom &g, int b0, double tprime) {
     pt.start(g, b0, tprime);
-    sincos_2pi((double)(long long)pt.d * 0x1p-64, &ds, &dc);
   }
   __device__ __forceinline__ void plane(int j) {
-    if ((j & 7) == 0) {
-      sincos_2pi(pt.turns_f64(j), &s, &c);
-    } else {
-      const double r = c * dc - s * ds;
-      s = s * dc + c * ds;
-      c = r;
-    }
+    const unsigned long long ph = pt.a + (unsigned long long)(unsigned)j * pt.d;
+    const unsigned m = (unsigned)((ph + (1ull << 55)) >> 56);  // the last half step is m = 0's
+    const double r = (double)(long long)(ph - ((unsigned long long)m << 56)) *
+                     (6.2831853071795864769 * 0x1p-64);
+    const double r2 = r * r;
+    const double sn = fma(r, r2 * fma(r2, 1.0 / 120.0, -1.0 / 6.0), r);
+    const double cm1 = r2 * fma(r2, fma(r2, -1.0 / 720.0, 1.0 / 24.0), -0.5);
+    const double2 w = tab[m & (kTurnTable - 1)];
+    c = w.x + fma(w.x, cm1, -(w.y * sn));
+    s = w.y + fma(w.y, cm1, w.x * sn);
   }
 };
+
+// The table that PlaneScreen<R> reads (every thread of the block calls it).
+template <typename R> __device__ __forceinline__ const double2 *screen_table() {
+  return nullptr;
+}
+template <> __device__ __forceinline__ const double2 *screen_table<double>() {
+  __shared__ double2 tab[kTurnTable];
+  turn_table(tab);
+  __syncthreads();
+  return tab;
+}
 
 // ---------------------------------------------------------------------
 // Tile kernels: lane map and shared-memory layout.

@@ -539,13 +539,14 @@ __global__ void __launch_bounds__(kThreads)
   const int ox = (g.ngx - g.nx) / 2, oy = (g.ngy - g.ny) / 2;
   const size_t plane = (size_t)g.ngx * g.ngy;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const double2 *tab = screen_table<R>();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < npix; i += stride) {
     const int iy = (int)(i / g.nx), ix = (int)(i - (int64_t)iy * g.nx);
     R a[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) a[p] = first ? (R)0 : acc[p * npix + i];
     const size_t gi = (size_t)(iy + oy) * g.ngx + (ix + ox);
-    PlaneScreen<R> ps;
+    PlaneScreen<R> ps(tab);
     ps.start(g, b0, tprime[i]);
     for (int j = 0; j < nb; ++j) {
       ps.plane(j);

@@ -65,13 +65,14 @@ __global__ void __launch_bounds__(kThreads)
   const int64_t npix = (int64_t)g.nx * g.ny, plane = (int64_t)g.ngx * g.ngy;
   const int ox = (g.ngx - g.nx) / 2, oy = (g.ngy - g.ny) / 2;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const double2 *tab = g.do_w ? screen_table<R>() : nullptr;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < npix; i += stride) {
     const int iy = (int)(i / g.nx), ix = (int)(i - (int64_t)iy * g.nx);
     C *dst = grid + (int64_t)(iy + oy) * g.ngx + ix + ox;
     R v[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) v[p] = img[p * npix + i];
-    PlaneScreen<R> ps;
+    PlaneScreen<R> ps(tab);
     if (g.do_w) ps.start(g, b0, tprime[i]);
     for (int j = 0; j < nb; ++j) {
       if (g.do_w) {
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(kThreads)
   const int ox = (g.ngx - g.nx) / 2, oy = (g.ngy - g.ny) / 2;
   const int64_t plane = (int64_t)g.ngx * g.ngy;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const double2 *tab = g.do_w ? screen_table<R>() : nullptr;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < plane; i += stride) {
     const int my = (int)(i / g.ngx), mx = (int)(i - (int64_t)my * g.ngx);
     const int ix = mx - ox, iy = my - oy;
@@ -109,7 +111,7 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
       for (int p = 0; p < NP; ++p) v[p] = img[p * npix + pi];
       if (g.do_w) {
-        PlaneScreen<R> ps;
+        PlaneScreen<R> ps(tab);
         ps.start(g, b0, tprime[pi]);
         for (int j = 0; j < nb; ++j) {
           ps.plane(j);
