@@ -51,6 +51,12 @@ def shape_key(npix_x, npix_y, pixsize_x, npol, precision, epsilon, do_wstacking,
         "%.3g" % float(epsilon), int(bool(do_wstacking)), int(nrows), int(nchan)))
 
 
+def _form(key):
+    """The precision named in a :func:`shape_key` (None in any other key)."""
+    parts = key.split("|")
+    return parts[4] if len(parts) == 9 else None
+
+
 def _load():
     if _loaded[0]:
         return
@@ -139,7 +145,8 @@ def autotune(key, run, start=None, candidates=None, max_seconds=120.0, repeats=1
     every timing.
 
     :param start: the planner's own choice (sigma, tile, slab, planes as a
-        plan reported them); the search starts from it and varies one
+        plan reported them); the search starts from it (in the FP64 form also
+        with sigma 0, the planner's own grid) and varies one
         parameter at a time: sigma over SIGMAS, tile over TILES, slab over
         SLABS, planes per batch over half / double the start (kept below
         ``max_batch_bytes`` when ``plane_bytes``, one plane's grid bytes at
@@ -172,6 +179,10 @@ def autotune(key, run, start=None, candidates=None, max_seconds=120.0, repeats=1
         if start is None:
             raise ValueError("autotune needs the planner's choice (start) or candidates")
         base = {k: start[k] for k in PARAMS}
+        if _form(key) == "fp64":
+            # sigma 0 is the planner's own plan: at an oversampling of its choice it
+            # may raise the grid sides to powers of two, which a given one's never are
+            consider(dict(base, sigma=0.0))
         consider(base)
         options = {"sigma": SIGMAS, "tile": TILES, "slab": SLABS}
         pl = int(base["planes"])
