@@ -1,12 +1,16 @@
 // Predict (dirty2ms): model image -> visibilities.
 //
 // Per call:   k_prep_image  image * correction, into [pol][y][x] order.
-// Per batch of w-planes:
-//             k_screen_pad  every grid cell of every plane in the batch is
-//                           written once: the central block gets
-//                           image * exp(+2 pi i w_k (n-1-tc)), the rest 0
-//                           (no separate memset pass).
-//             cuFFT         2-D c2c, e^{-2 pi i}
+// Per batch of w-planes, one of
+//             columns, rows (FP32 form, gb_fft.cu and gb_rows.cu) the screens
+//                           image * exp(+2 pi i w_k (n-1-tc)) fused into the
+//                           columns' first step; occupied bins written;
+//             k_screen_block, k_fft64 (FP64 form, gb_fft64.cu) the screened
+//                           image, then its transform; occupied bins written;
+//             k_screen_pad, cuFFT every grid cell of every plane written once,
+//                           the central block screened, the rest 0 (no separate
+//                           memset pass); 2-D c2c, e^{-2 pi i}.
+//             Then
 //             k_degrid_warp one CTA per work chunk (FP32 form): every item's
 //                           kernel values cached once per chunk; supports
 //                           of up to 7 cells from planes staged in shared
@@ -437,8 +441,8 @@ template <int NV> __device__ __forceinline__ void reduce8(float *v, int lane) {
   for (int o = 4 / NV; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
 }
 
-// Chunks of few items, supports of up to 7 cells: a warp per item over all its
-// planes, the cells of a 7 x 7 frame dealt to the lanes (two each), their weights
+// Chunks of few items, supports of up to 7 cells, with w-stacking (as every staged
+// plan): a warp per item over all its planes, the cells of a 7 x 7 frame dealt to the lanes (two each), their weights
 // and offsets formed once and the planes' cells read straight from the grid with
 // no wait between planes; one reduction per item.
 template <int NP>
@@ -448,7 +452,7 @@ __device__ __forceinline__ void degrid_sparse_chunk(
     const float *__restrict__ wgt, const PolMat &pm, const RowPerm &rp, float2 *sacc) {
   constexpr int NV = 2 * NP;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int W = g.W, T = g.T, wk = g.do_w ? W : 1, n = (int)(ch.end - ch.begin);
+  const int W = g.W, T = g.T, n = (int)(ch.end - ch.begin);
   const int ntiles = g.ntu * g.ntv;
   const int64_t plane = (int64_t)g.ngx * g.ngy;
   const int slab = (int)(ch.bucket / (uint32_t)ntiles);
@@ -459,11 +463,10 @@ __device__ __forceinline__ void degrid_sparse_chunk(
     const ItemF it = items[ch.begin + jj];
     const int lu = (int)(it.loc & 0xffu), lv = (int)((it.loc >> 8) & 0xffu);
     const int k0 = kbase + (int)((it.loc >> 16) & 0xffu);
-    const int k_lo = max(k0, b0), k_hi = min(k0 + wk, b0 + nb);
+    const int k_lo = max(k0, b0), k_hi = min(k0 + W, b0 + nb);
     const float d = dim == 0 ? it.du : (dim == 1 ? it.dv : it.dwf);
     float val = 0.f;
-    if (dim < 3 && a_k < W)
-      val = dim == 2 && !g.do_w ? 1.f : es_kernel(((float)a_k - d) * (2.f / (float)W), (float)g.beta);
+    if (dim < 3 && a_k < W) val = es_kernel(((float)a_k - d) * (2.f / (float)W), (float)g.beta);
     float2 w[2];
     int64_t off[2];
 #pragma unroll
@@ -530,7 +533,7 @@ __device__ __forceinline__ void degrid_staged_chunk(
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float scale_u = 2.f / (float)W, beta = (float)g.beta;
-  const int ntiles = g.ntu * g.ntv, wk = g.do_w ? W : 1;
+  const int ntiles = g.ntu * g.ntv;
   const int64_t plane = (int64_t)g.ngx * g.ngy;
   const int slab = (int)(ch.bucket / (uint32_t)ntiles);
   const int tile = (int)(ch.bucket - (uint32_t)slab * ntiles);
@@ -541,7 +544,7 @@ __device__ __forceinline__ void degrid_staged_chunk(
   const int lk_first = (int)((items[ch.begin].loc >> 16) & 0xffu);
   const int lk_last = (int)((items[ch.end - 1].loc >> 16) & 0xffu);
   const int k_lo = max(kbase + lk_first, b0);
-  const int k_hi = min(min(kbase + lk_last + wk, g.nplanes), b0 + nb);
+  const int k_hi = min(min(kbase + lk_last + W, g.nplanes), b0 + nb);
   if (k_lo >= k_hi) return;  // (block-uniform) no item reaches this batch's planes
   for (int i = threadIdx.x; i < SW; i += NT) {
     int q = tv * T + i;
@@ -591,8 +594,7 @@ __device__ __forceinline__ void degrid_staged_chunk(
     float *k = c + 2 + 8 * dim;
 #pragma unroll
     for (int a = 0; a < 7; ++a) {
-      float x = a < W ? es_kernel(((float)a - d) * scale_u, beta) : 0.f;
-      if (dim == 2 && !g.do_w) x = 1.f;
+      const float x = a < W ? es_kernel(((float)a - d) * scale_u, beta) : 0.f;
       k[a] = dim < 2 && ((first + a) & 1) ? -x : x;
     }
     if (dim < 2) k[7] = 0.f;
@@ -629,7 +631,7 @@ __device__ __forceinline__ void degrid_staged_chunk(
     __syncthreads();  // window staged (and, first, the item cache written)
     const int np = k_next - k;
     // items whose support reaches a plane of the window
-    const int lk_lo = max(0, k - kbase - wk + 1), lk_hi = min(g.S - 1, k + np - 1 - kbase);
+    const int lk_lo = max(0, k - kbase - W + 1), lk_hi = min(g.S - 1, k + np - 1 - kbase);
     const int jlo = s_first[min(lk_lo, g.S)], jhi = lk_lo <= lk_hi ? s_first[lk_hi + 1] : jlo;
     const float4 *win = sheets + (size_t)buf * kStageSheets * SW * hp;
     for (int j0 = jlo + 4 * warp; j0 < jhi; j0 += 4 * kStageWarps) {
@@ -656,7 +658,7 @@ __device__ __forceinline__ void degrid_staged_chunk(
         if (q < np) {  // block-uniform
           // a plane of the chunk that this item does not reach weighs 0
           const int aw = aw0 + q;
-          const float kw = aw >= 0 && aw < wk ? kj[18 + aw] : 0.f;
+          const float kw = aw >= 0 && aw < W ? kj[18 + aw] : 0.f;
           const float2 kw2 = make_float2(kw, kw);
 #pragma unroll
           for (int p = 0; p < NP; ++p) {
