@@ -116,7 +116,9 @@ typedef struct {
   int32_t support, ngrid_x, ngrid_y, nplanes, planes_per_batch, tile, slab;
   double beta, sigma, dw, w_lo, w_hi, tc;
   int64_t nitems, nbuckets, workspace_bytes;
-  int32_t fft_mode;    /* the gb_fft_mode in use (never GB_FFT_AUTO)           */
+  int32_t fft_mode;    /* the gb_fft_mode in use (never GB_FFT_AUTO); GB_FFT_CUFFT_2D
+                          also where GB_FFT_AUTO came to the FP64 form's own 2-D
+                          transforms                                          */
   int32_t own_rows;    /* 1: GB_FFT_COLUMNS with the library's row transforms
                           (grid width a power of two from 512 to 16384: no
                           cuFFT plan, cells without visibilities skipped);

@@ -134,7 +134,7 @@ __device__ __forceinline__ double2 exp_turns(double d, const TurnScale &s, const
 // by FP64 instructions: 3 for the row and component, 30 for the two exponentials,
 // 18 for the eight channels and 4 per channel and pol for the sum.  65,024 rows x 8
 // channels x 200 components x 1 pol: 3.9 ms with two sincospi and successive
-// products in blocks of 256 threads (two waves of blocks on 152 SMs), 2.4 ms so, in
+// products in blocks of 256 threads (two waves of blocks on 152 SMs), 2.6 ms so, in
 // blocks of 64.
 constexpr int kDftThreads = 64;
 

@@ -125,6 +125,9 @@ static bool fft64_applies(const gb_plan_params *p, const Geom &g) {
 // 4.3e-11 at 2048^2).
 constexpr double kCostCell64Cufft = 1.8e-10, kCostCell64Own = 6.0e-11;
 
+// Padded grids at this epsilon and below.  Not a limit of accuracy (the larger grid
+// keeps epsilon too): another grid gives another aliasing error, so it moves a
+// result by up to epsilon (1e-7 seen at 1e-6), and below 1e-9 nobody sees that.
 constexpr double kPadEpsilon = 1e-9;
 
 static int next_pow2(int n) {
@@ -169,9 +172,7 @@ int plan_geometry(const gb_plan_params *p, double w_lo, double w_hi, Geom &g) {
   if (!found) return plan_geometry_sigma(p, w_lo, w_hi, 2.0, g);  // for its error message
   // the FP64 form at that oversampling: sides raised to powers of two where the
   // library's own transforms of the larger grid cost less than cuFFT's of the
-  // smaller (the wider oversampling only lowers the aliasing error).  Another grid
-  // moves the result by up to epsilon: only where that is at the level FP64
-  // results are compared at
+  // smaller (the wider oversampling only lowers the aliasing error)
   if (p->precision == GB_FP64 && p->epsilon <= kPadEpsilon && p->fft_mode == GB_FFT_AUTO &&
       !fft64_applies(p, g)) {
     Geom t;

@@ -60,7 +60,9 @@ class Plan:
     :param fft_mode: "auto" (the library's column kernels where they apply:
         FP32 form, power-of-two grid height), "columns" (require them) or
         "cufft2d" (batched 2-D cuFFT plans); ``info["fft_mode"]`` reports
-        the one in use (2 = columns, 1 = cufft2d)
+        the one in use (2 = columns, 1 = 2-D transforms: cuFFT's, or under
+        "auto" in the FP64 form on power-of-two grids from 128 to 4096 that
+        are twice the image or more, the library's own)
     :param sigma: grid oversampling (1.25, 1.5, 1.75, 2); 0 = the planner's
         choice by its cost model (or a cached autotuning result)
     :param planes_per_batch: w-planes per transform batch (0: what
